@@ -21,10 +21,11 @@ LIBDIR = PKG / "_lib"
 LIB = LIBDIR / "libgb300kf.so"
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["kf_capi.cu", "kf_fit_fp64.cu", "kf_fit_mixed.cu", "kf_fit_fp64_mat.cu",
-              "kf_fit_mixed_mat.cu", "kf_batch.cu", "kf_diag.cu",
-              "kf_noalloc.cu", "kf_adjoint.cu", "kf_sim.cu"] + [f"kf_tune_{p}_{m}.cu" for p in ("fp64", "mixed")
-                                                     for m in ("2", "3", "5", "64x4", "64x8", "256x1", "256x2")]
+# fit kernels: one file per precision and register budget
+CU_SOURCES = ["kf_capi.cu", "kf_launch.cu", "kf_batch.cu", "kf_fit_material.cu",
+              "kf_fit_material_states.cu", "kf_diag.cu", "kf_noalloc.cu", "kf_adjoint.cu",
+              "kf_sim.cu"] + [f"kf_fit_{p}_{r}.cu" for p in ("fp64", "mixed")
+                              for r in (255, 168, 128, 96)]
 CXX_SOURCES = ["synth.cpp", "kf_io.cpp", "kf_fieldmap.cpp"]
 # The simulation kernel runs the host generator's per-track code; without
 # contraction into FMA on either side the two differ only by the math

@@ -33,7 +33,6 @@
 
 #include "kf_adjoint_math.h"
 #include "kf_host.h"
-#include "kf_kernels.cuh"
 
 using namespace kfh;
 

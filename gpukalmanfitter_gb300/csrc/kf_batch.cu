@@ -16,98 +16,11 @@
 #include <new>
 
 #include "kf_host.h"
-#include "kf_kernels.cuh"
 
 using namespace kfd;
 using namespace kfh;
 
-// persistent-kernel instantiations (kf_fit_*.cu, kf_tune_*.cu): launcher and
-// shared-memory set-up
-cudaError_t launchPersistent_fp64_128_4(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_128_4_prep();
-cudaError_t launchPersistent_fp64_128_2(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_128_2_prep();
-cudaError_t launchPersistent_fp64_128_3(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_128_3_prep();
-cudaError_t launchPersistent_fp64_128_5(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_128_5_prep();
-cudaError_t launchPersistent_fp64_64_4(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_64_4_prep();
-cudaError_t launchPersistent_fp64_64_8(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_64_8_prep();
-cudaError_t launchPersistent_fp64_256_1(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_256_1_prep();
-cudaError_t launchPersistent_fp64_256_2(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_256_2_prep();
-cudaError_t launchPersistent_mixed_128_4(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_128_4_prep();
-cudaError_t launchPersistent_mixed_128_2(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_128_2_prep();
-cudaError_t launchPersistent_mixed_128_3(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_128_3_prep();
-cudaError_t launchPersistent_mixed_128_5(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_128_5_prep();
-cudaError_t launchPersistent_mixed_64_4(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_64_4_prep();
-cudaError_t launchPersistent_mixed_64_8(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_64_8_prep();
-cudaError_t launchPersistent_mixed_256_1(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_256_1_prep();
-cudaError_t launchPersistent_mixed_256_2(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_256_2_prep();
-cudaError_t launchPersistent_fp64_mat(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_fp64_mat_prep();
-cudaError_t launchPersistent_mixed_mat(const kfd::Params &, cudaStream_t);
-cudaError_t launchPersistent_mixed_mat_prep();
-
 namespace {
-
-struct Variant {
-  int precision, bs, minb;
-  cudaError_t (*launch)(const Params &, cudaStream_t);
-  cudaError_t (*prep)();
-};
-// (threads per CTA, CTAs per SM): register budgets 255 (128x2, 64x4, 256x1),
-// 168 (128x3), 128 (128x4, 64x8, 256x2), 96 (128x5)
-const Variant kVariants[] = {
-    {KF_PRECISION_FP64, 128, 4, launchPersistent_fp64_128_4, launchPersistent_fp64_128_4_prep},
-    {KF_PRECISION_FP64, 128, 2, launchPersistent_fp64_128_2, launchPersistent_fp64_128_2_prep},
-    {KF_PRECISION_FP64, 128, 3, launchPersistent_fp64_128_3, launchPersistent_fp64_128_3_prep},
-    {KF_PRECISION_FP64, 128, 5, launchPersistent_fp64_128_5, launchPersistent_fp64_128_5_prep},
-    {KF_PRECISION_FP64, 64, 4, launchPersistent_fp64_64_4, launchPersistent_fp64_64_4_prep},
-    {KF_PRECISION_FP64, 64, 8, launchPersistent_fp64_64_8, launchPersistent_fp64_64_8_prep},
-    {KF_PRECISION_FP64, 256, 1, launchPersistent_fp64_256_1, launchPersistent_fp64_256_1_prep},
-    {KF_PRECISION_FP64, 256, 2, launchPersistent_fp64_256_2, launchPersistent_fp64_256_2_prep},
-    {KF_PRECISION_MIXED, 128, 4, launchPersistent_mixed_128_4, launchPersistent_mixed_128_4_prep},
-    {KF_PRECISION_MIXED, 128, 2, launchPersistent_mixed_128_2, launchPersistent_mixed_128_2_prep},
-    {KF_PRECISION_MIXED, 128, 3, launchPersistent_mixed_128_3, launchPersistent_mixed_128_3_prep},
-    {KF_PRECISION_MIXED, 128, 5, launchPersistent_mixed_128_5, launchPersistent_mixed_128_5_prep},
-    {KF_PRECISION_MIXED, 64, 4, launchPersistent_mixed_64_4, launchPersistent_mixed_64_4_prep},
-    {KF_PRECISION_MIXED, 64, 8, launchPersistent_mixed_64_8, launchPersistent_mixed_64_8_prep},
-    {KF_PRECISION_MIXED, 256, 1, launchPersistent_mixed_256_1, launchPersistent_mixed_256_1_prep},
-    {KF_PRECISION_MIXED, 256, 2, launchPersistent_mixed_256_2, launchPersistent_mixed_256_2_prep},
-};
-
-// with material effects: the one instantiation with the material code
-// (128 threads, 4 CTAs per SM), whatever the shape fields say
-const Variant kMaterialVariants[] = {
-    {KF_PRECISION_FP64, 128, 4, launchPersistent_fp64_mat, launchPersistent_fp64_mat_prep},
-    {KF_PRECISION_MIXED, 128, 4, launchPersistent_mixed_mat, launchPersistent_mixed_mat_prep},
-};
-
-// the instantiation for a configuration (block size 0/128, min blocks 0 = 4)
-const Variant *findVariant(const kf_config_t *cfg) {
-  if (cfg->material_effects) {
-    for (const Variant &v : kMaterialVariants)
-      if (v.precision == cfg->precision) return &v;
-    return nullptr;
-  }
-  const int bs = cfg->block_size ? cfg->block_size : 128;
-  const int mb = cfg->min_blocks_per_sm ? cfg->min_blocks_per_sm : 4;
-  for (const Variant &v : kVariants)
-    if (v.precision == cfg->precision && v.bs == bs && v.minb == mb) return &v;
-  return nullptr;
-}
 
 constexpr int kBuckets = kSortBuckets;
 
@@ -190,7 +103,7 @@ int32_t kfh::sortQueue(const Params &P, int32_t *hist, int32_t *offs, int32_t *p
 
 namespace {
 
-int32_t enqueueBatched(const Params &P, const Variant *v, char *base, const BatchLayout &L,
+int32_t enqueueBatched(Params &P, const kf_config_t *cfg, char *base, const BatchLayout &L,
                        cudaStream_t s) {
   if (P.n == 0) return KF_SUCCESS;
   HostRange range("work-queue sort + persistent fit");
@@ -200,14 +113,14 @@ int32_t enqueueBatched(const Params &P, const Variant *v, char *base, const Batc
                                reinterpret_cast<int32_t *>(base + L.offs),
                                reinterpret_cast<int32_t *>(base + L.perm), s);
   if (rc) return rc;
-  e = v->launch(P, s);
+  e = launchFit(P, cfg->precision, cfg->block_size, cfg->min_blocks_per_sm, s);
   if (e != cudaSuccess) return cudaFail(e, "persistent fit launch");
   return KF_SUCCESS;
 }
 
 int32_t prepare(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t *cfg,
                 const kf_geometry_t *geo, const kf_field_t *field, void *workspace,
-                size_t bytes, Params &P, const Variant *&v, BatchLayout &L) {
+                size_t bytes, Params &P, BatchLayout &L) {
   int32_t rc = checkCommon(in, cfg, geo, field);
   if (rc) return rc;
   if (!out || !out->params || !out->cov || !out->chi2 || !out->status || !out->n_meas)
@@ -216,12 +129,9 @@ int32_t prepare(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t *cfg
     return fail(KF_ERR_INVALID_ARGUMENT, "missing input array%s");
   // the int32 queue counter runs up to n + 32 x (resident warps)
   if (in->n_tracks > 0x7f000000LL) return fail(KF_ERR_INVALID_ARGUMENT, "batch above 2^31 - 2^24 tracks%s");
-  v = findVariant(cfg);
-  if (!v) return fail(KF_ERR_UNSUPPORTED, "no persistent kernel for this block size / CTAs per SM%s");
-  {
-    const cudaError_t e = v->prep();
-    if (e != cudaSuccess) return cudaFail(e, "persistent kernel shared-memory set-up");
-  }
+  // with material effects there is one shape, whatever the fields say
+  if (!cfg->material_effects && !shapeCompiled(cfg->block_size, cfg->min_blocks_per_sm))
+    return fail(KF_ERR_UNSUPPORTED, "no persistent kernel for this block size / CTAs per SM%s");
   L = batchLayout(in->n_tracks, in->n_surfaces, cfg->material_effects != 0);
   if (in->n_tracks > 0 && (!workspace || bytes < L.total))
     return fail(KF_ERR_WORKSPACE_TOO_SMALL, "workspace smaller than kf_batch_workspace_size()%s");
@@ -251,11 +161,10 @@ int32_t kf_fit_batch_sorted(const kf_inputs_t *in, kf_outputs_t *out, const kf_c
                             const kf_geometry_t *geo, const kf_field_t *field, void *workspace,
                             size_t workspace_bytes, void *stream) {
   Params P;
-  const Variant *v = nullptr;
   BatchLayout L;
-  int32_t rc = prepare(in, out, cfg, geo, field, workspace, workspace_bytes, P, v, L);
+  int32_t rc = prepare(in, out, cfg, geo, field, workspace, workspace_bytes, P, L);
   if (rc) return rc;
-  return enqueueBatched(P, v, static_cast<char *>(workspace), L, static_cast<cudaStream_t>(stream));
+  return enqueueBatched(P, cfg, static_cast<char *>(workspace), L, static_cast<cudaStream_t>(stream));
 }
 
 int32_t kf_batch_plan_create(kf_batch_plan_t **plan, const kf_inputs_t *in, kf_outputs_t *out,
@@ -266,14 +175,13 @@ int32_t kf_batch_plan_create(kf_batch_plan_t **plan, const kf_inputs_t *in, kf_o
   *plan = nullptr;
   if (!stream) return fail(KF_ERR_INVALID_ARGUMENT, "a plan needs a created stream (not the legacy default stream)%s");
   Params P;
-  const Variant *v = nullptr;
   BatchLayout L;
-  int32_t rc = prepare(in, out, cfg, geo, field, workspace, workspace_bytes, P, v, L);
+  int32_t rc = prepare(in, out, cfg, geo, field, workspace, workspace_bytes, P, L);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cudaFail(e, "stream capture begin");
-  rc = enqueueBatched(P, v, static_cast<char *>(workspace), L, s);
+  rc = enqueueBatched(P, cfg, static_cast<char *>(workspace), L, s);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s, &graph);
   if (rc) {
@@ -330,14 +238,13 @@ int32_t kf_autotune(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t 
   double best = 1e300;
   kf_config_t bestCfg = *cfg;
   int32_t rc = KF_SUCCESS;
-  for (const Variant &v : kVariants) {
-    if (v.precision != cfg->precision) continue;
-    // with material effects the one material instantiation (128 x 4) runs
-    if (cfg->material_effects && (v.bs != 128 || v.minb != 4)) continue;
+  int bs = 0, minb = 0;
+  // with material effects there is one shape
+  for (int v = 0; fitShape(v, &bs, &minb) && (v == 0 || !cfg->material_effects); ++v) {
     kf_config_t c = *cfg;
     c.kernel = KF_KERNEL_PERSISTENT;
-    c.block_size = v.bs;
-    c.min_blocks_per_sm = v.minb;
+    c.block_size = bs;
+    c.min_blocks_per_sm = minb;
     rc = kf_fit_batch_sorted(&sample, out, &c, geo, field, workspace, workspace_bytes, stream);
     // best of three timed runs after one warm-up
     for (int r = 0; r < 3 && rc == KF_SUCCESS; ++r) {

@@ -13,16 +13,8 @@
 #include <mutex>
 
 #include "kf_host.h"
-#include "kf_kernels.cuh"
 
 using namespace kfd;
-
-// defined in kf_fit_fp64.cu / kf_fit_mixed.cu (one instantiation each, so the
-// two compile in parallel)
-cudaError_t launchFitFp64(const kfd::Params &P, unsigned grid, cudaStream_t s);
-cudaError_t launchFitMixed(const kfd::Params &P, unsigned grid, cudaStream_t s);
-cudaError_t launchFitFp64Mat(const kfd::Params &P, unsigned grid, cudaStream_t s);
-cudaError_t launchFitMixedMat(const kfd::Params &P, unsigned grid, cudaStream_t s);
 
 namespace {
 thread_local char g_err[512] = "";
@@ -122,6 +114,7 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
       F.invw[a] = (field->kind == KF_FIELD_GRID_RZ && a == 1)
                       ? 0.
                       : (na - 1) / (field->max[a] - field->min[a]);
+      F.off[a] = -F.mn[a] * F.invw[a] - 0.5;
     }
   }
   F.grid = reinterpret_cast<const float4 *>(field->grid);
@@ -135,6 +128,8 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
   F.scalef = (float)F.scale;
   F.scalelo = (float)(F.scale - (double)F.scalef);
   P.tolLoF = (float)(P.tol * 0.99);
+  // below the reference's floor of the error estimate (1e-20) FP64 decides
+  P.tolAcceptF = P.tol > 1e-19 ? (float)(P.tol * (1. - 1e-5)) : -1.f;
   for (int k = 0; k < in->n_surfaces; ++k) {
     PlaneD &pl = P.planes[k];
     for (int r = 0; r < 3; ++r) {
@@ -159,23 +154,6 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
 } // namespace kfh
 
 using namespace kfh;
-
-namespace {
-
-int32_t launchFit(const Params &P, int precision, int blockSize, cudaStream_t s) {
-  (void)blockSize;
-  if (P.n == 0) return KF_SUCCESS;
-  const unsigned grid = (unsigned)((P.n + kFitBlock - 1) / kFitBlock);
-  const bool mat = P.materialEffects != 0;
-  cudaError_t e = (precision == KF_PRECISION_MIXED)
-                      ? (mat ? launchFitMixedMat(P, grid, s) : launchFitMixed(P, grid, s))
-                      : (mat ? launchFitFp64Mat(P, grid, s) : launchFitFp64(P, grid, s));
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) return cudaFail(e, "fit kernel launch");
-  return KF_SUCCESS;
-}
-
-} // namespace
 
 extern "C" {
 
@@ -221,7 +199,9 @@ int32_t kf_fit_batch(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t
     return fail(KF_ERR_WORKSPACE_TOO_SMALL, "workspace smaller than kf_workspace_size()%s");
   Params P;
   fillParams(P, in, out, cfg, geo, field, workspace);
-  return launchFit(P, cfg->precision, cfg->block_size, static_cast<cudaStream_t>(stream));
+  if (P.n == 0) return KF_SUCCESS;
+  const cudaError_t e = launchFit(P, cfg->precision, 0, 0, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
 }
 
 // ---- host-buffer convenience ----------------------------------------------

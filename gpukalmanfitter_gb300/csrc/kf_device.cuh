@@ -61,7 +61,7 @@ struct FieldD {
   int n[3];
   double B[3]; // constant field, scale applied
   double scale;
-  double mn[3], invw[3];
+  double mn[3], invw[3], off[3]; // off = -mn invw - 1/2
   const float4 *grid;
   float Bf[3], mnf[3], invwf[3], scalef; // FP32 copies for the mixed form
   float Blo[3], wf[3], scalelo;          // mixed form: lo parts of B and scale, cell width
@@ -73,6 +73,7 @@ struct Params {
   int maxSteps, maxTrials, smoothing, faithful;
   double tol, cutoff, mass, overstep, surfTol, outlierCut;
   float tolLoF;         // mixed form: FP32 error estimates up to this accept
+  float tolAcceptF;     // FP64 forms: FP32-rounded error estimates up to this accept
   const double *meas;
   const uint64_t *mask;
   const int32_t *nplanes;
@@ -85,6 +86,11 @@ struct Params {
                          // covariance per state (the general smoother's input)
   const int32_t *perm;   // batched form: queue position -> track index
   int32_t *queueCounter; // batched form: next unclaimed queue position
+  // FP64 fit in a uniform field: the field along z of the frame that the
+  // planes are given in (rot: its axes, rows; the identity unless rotated)
+  double Bz, rot[9];
+  float rotf[9];
+  int rotated;
   FieldD field;
   PlaneD planes[KF_MAX_PLANES];
   kfm::Slab planeSlab[KF_MAX_PLANES]; // surface material (kf_geometry_t.material)
@@ -376,7 +382,7 @@ __device__ __forceinline__ long long okey(double x) {
 __device__ __forceinline__ long long akey(double x) {
   return __double_as_longlong(x) & 0x7fffffffffffffffLL;
 }
-template <typename R, typename H> __device__ __forceinline__ double ssMax(const Lane<R, H> &L) {
+template <class LT> __device__ __forceinline__ double ssMax(const LT &L) {
   double m = L.ss[0];
   long long km = okey(m);
 #pragma unroll
@@ -389,7 +395,7 @@ template <typename R, typename H> __device__ __forceinline__ double ssMax(const 
   }
   return m;
 }
-template <typename R, typename H> __device__ __forceinline__ double ssMin(const Lane<R, H> &L) {
+template <class LT> __device__ __forceinline__ double ssMin(const LT &L) {
   double m = L.ss[0];
   long long km = okey(m);
 #pragma unroll
@@ -402,18 +408,18 @@ template <typename R, typename H> __device__ __forceinline__ double ssMin(const 
   }
   return m;
 }
-template <typename R, typename H> __device__ __forceinline__ double ssValue(const Lane<R, H> &L) {
+template <class LT> __device__ __forceinline__ double ssValue(const LT &L) {
   return L.ssDir == 1 ? ssMin(L) : ssMax(L);
 }
-template <typename R, typename H> __device__ __forceinline__ void ssRelease(Lane<R, H> &L, int t) {
+template <class LT> __device__ __forceinline__ void ssRelease(LT &L, int t) {
   L.ss[t] = (L.ssDir == 1) ? ssMax(L) : ssMin(L);
 }
-template <typename R, typename H> __device__ __forceinline__ void ssUpdate(Lane<R, H> &L, double v, int t, bool rel) {
+template <class LT> __device__ __forceinline__ void ssUpdate(LT &L, double v, int t, bool rel) {
   if (rel) ssRelease(L, t);
   const double c = L.ss[t];
   L.ss[t] = akey(c) < akey(v) ? c : v;
 }
-template <typename R, typename H> __device__ __forceinline__ void ssInit(Lane<R, H> &L, double value) {
+template <class LT> __device__ __forceinline__ void ssInit(LT &L, double value) {
   L.ssDir = value > 0. ? 1 : -1;
   L.ss[0] = DBL_MAX * L.ssDir;
   L.ss[1] = DBL_MAX * L.ssDir;
@@ -683,8 +689,8 @@ __device__ __forceinline__ float rkTrialDelta(const FieldD &F, const float pos[3
   return (e < 1e-20f) ? 1e-20f : e;
 }
 
-template <typename R, typename H>
-__device__ __forceinline__ void applyTransportStep(Lane<R, H> &L, const R DA[3][3], const R DB[3][3],
+template <typename R, class LT>
+__device__ __forceinline__ void applyTransportStep(LT &L, const R DA[3][3], const R DB[3][3],
                                                    const R Da[3], const R Dc[3], R D37);
 
 // The mixed form's J = D J on offsets from the straight line: with
@@ -692,8 +698,8 @@ __device__ __forceinline__ void applyTransportStep(Lane<R, H> &L, const R DA[3][
 //   dA' = dA + h dB + dDA (I + dB),  a' = a + h c + dDA c + Da,
 //   dB' = dB + dDB (I + dB),         c' = c + dDB c + Dc,   b' = b + D37,
 // every FP32 term a field-induced quantity (the path s is advanced in FP64).
-template <typename R, typename H>
-__device__ __forceinline__ void applyTransportOffsets(Lane<R, H> &L, R h, const R dDA[3][3],
+template <typename R, class LT>
+__device__ __forceinline__ void applyTransportOffsets(LT &L, R h, const R dDA[3][3],
                                                       const R dDB[3][3], const R Da[3],
                                                       const R Dc[3], R D37) {
   R nA[3][3], na[3], nB[3][3], nc[3];
@@ -724,8 +730,8 @@ __device__ __forceinline__ void applyTransportOffsets(Lane<R, H> &L, R h, const 
 
 // transportMatrix (EigenStepper.ipp:50-124) on its non-zero blocks and
 // jacTransport = D * jacTransport (EigenStepper.ipp:312-318)
-template <typename R, typename H>
-__device__ __forceinline__ void transportUpdate(Lane<R, H> &L, const R dir[3], R qop, R h, R d37,
+template <typename R, class LT>
+__device__ __forceinline__ void transportUpdate(LT &L, const R dir[3], R qop, R h, R d37,
                                                 const RkStages<R> &s) {
   const R half_h = h * R(0.5);
   R dk1dL[3], dk2dL[3], dk3dL[3], dk4dL[3], tmp[3], c[3], cc[3];
@@ -797,8 +803,8 @@ __device__ __forceinline__ void transportUpdate(Lane<R, H> &L, const R dir[3], R
 }
 
 // new J = D * J on the structured blocks (EigenStepper.ipp:312-318)
-template <typename R, typename H>
-__device__ __forceinline__ void applyTransportStep(Lane<R, H> &L, const R DA[3][3], const R DB[3][3],
+template <typename R, class LT>
+__device__ __forceinline__ void applyTransportStep(LT &L, const R DA[3][3], const R DB[3][3],
                                                    const R Da[3], const R Dc[3], R D37) {
   // new J = D * J:
   //  A' = A + DA*B,  a' = a + DA*c + Da,  b' = b + D37,
@@ -1722,156 +1728,6 @@ __device__ __forceinline__ void invJacobian(const T J[25], T Gi[25]) {
 }
 
 // ---------------------------------------------------------------------------
-// Actor::finalize (KalmanFitter.hpp:360-393) with the gain-matrix (RTS)
-// smoother (GainMatrixSmoother.hpp:21-94).  Returns false on a NaN gain.
-//
-// The reference gain is G = C_f J^T C_p'^-1 with C_p' = J C_f J^T the
-// predicted covariance of the next state.  On this path (no material, no
-// process noise) that product is exactly J^-1, and the smoothed covariance
-// C_s = C_f - G (C_p' - C_s') G^T reduces to G C_s' G^T.  The kernel uses
-// these closed forms: the same quantities in exact arithmetic, without the
-// cancellation of the reference form (whose q/p variance moves by 1e-9 to
-// 5e-8 relative between two valid FP64 evaluations), and without storing
-// covariances per state.
-// ---------------------------------------------------------------------------
-// Smoother when no smoothed-state output is requested: only the first
-// state's covariance leaves the fit, C_s(0) = Pg C_f(n-1) Pg^T with
-// Pg = G_1 ... G_{n-1} accumulated on the Jacobian structure (~190 instead of
-// ~470 FLOP per state for G C_s' G^T).  The gains G_i = J_i^-1 are formed in
-// T (FP32 in the mixed form, FP64 in the plain form); the corrections
-// J_i^-1 (x_s' - x_p') are FP64-accurate in both: the mixed form refines its
-// FP32 product once against the FP64 residual x_s' - x_p' - J_i y.
-template <typename T, typename R, typename H>
-__device__ bool finalizeSmoothGain(Lane<R, H> &L, const Params &P, const PlaneD *planes) {
-  L.smoothed = true;
-  const int n = L.measStates;
-  double xs[6];
-#pragma unroll
-  for (int e = 0; e < 6; ++e) xs[e] = *wsPtr(P, L, n - 1, 6 + e);
-  T Pg[25];
-#pragma unroll
-  for (int e = 0; e < 25; ++e) Pg[e] = (e < 20 && e % 6 == 0) ? T(1) : T(0); // rows 0..3: identity
-  for (int i = n - 2; i >= 0; --i) {
-    T Jn[25], G[25];
-#pragma unroll
-    for (int e = 0; e < 25; ++e) Jn[e] = (T)*wsPtr(P, L, i + 1, 12 + e);
-    invJacobian<T>(Jn, G);
-    bool nan = false;
-#pragma unroll
-    for (int e = 0; e < 25; ++e) nan = nan || (G[e] != G[e]);
-    if (nan) return false;
-    double dxd[6];
-#pragma unroll
-    for (int e = 0; e < 6; ++e) dxd[e] = xs[e] - *wsPtr(P, L, i + 1, e);
-    // y = G dx on the structure of J^-1
-    auto apply = [&](const double v[6], double out[6]) {
-      T dx[6];
-#pragma unroll
-      for (int e = 0; e < 6; ++e) dx[e] = (T)v[e];
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        if (r == 4) {
-          out[4] = (double)dx[4];
-        } else {
-          const int gr = (r == 5) ? 4 : r;
-          T g = G[5 * gr] * dx[0];
-#pragma unroll
-          for (int k = 1; k < 5; ++k) g += G[5 * gr + k] * dx[k];
-          if (r == 5) g += dx[5];
-          out[r] = (double)g;
-        }
-      }
-    };
-    double y[6];
-    apply(dxd, y);
-    if constexpr (sizeof(T) == sizeof(float)) {
-      // FP32 gain: one refinement step with the residual in FP64,
-      // r = dx - J y, y += G r, makes y = J^-1 dx to FP64 accuracy
-      double rd[6], y1[6];
-#pragma unroll
-      for (int r = 0; r < 6; ++r) {
-        if (r == 4) {
-          rd[4] = dxd[4] - y[4];
-        } else {
-          const int jr = (r == 5) ? 4 : r;
-          double v = dxd[r];
-#pragma unroll
-          for (int k = 0; k < 5; ++k) v -= *wsPtr(P, L, i + 1, 12 + 5 * jr + k) * y[k];
-          if (r == 5) v -= y[5];
-          rd[r] = v;
-        }
-      }
-      apply(rd, y1);
-#pragma unroll
-      for (int e = 0; e < 6; ++e) y[e] += y1[e];
-    }
-#pragma unroll
-    for (int e = 0; e < 6; ++e) xs[e] = *wsPtr(P, L, i, 6 + e) + y[e];
-    // Pg <- G Pg on the structure [[A, b, 0], [0, 1, 0], [c, d, 1]]
-    T Np[25];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        T v = G[5 * r] * Pg[c];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) v += G[5 * r + k] * Pg[5 * k + c];
-        if (c == 4) v += G[5 * r + 4];
-        if (r == 4) v += Pg[20 + c]; // row 5 of G times row 5 of Pg
-        Np[5 * r + c] = v;
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 25; ++e) Pg[e] = Np[e];
-  }
-  // C_s(0) = Pg C Pg^T with C the last filtered covariance (in the stepper)
-  double Cs[21];
-  {
-    double M[6][6];
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        if (r == 4) {
-          M[r][c] = L.cov(sidx(4, c));
-        } else {
-          const int gr = (r == 5) ? 4 : r;
-          double v = (double)Pg[5 * gr] * L.cov(sidx(0, c));
-#pragma unroll
-          for (int k = 1; k < 5; ++k) v += (double)Pg[5 * gr + k] * L.cov(sidx(k, c));
-          if (r == 5) v += L.cov(sidx(5, c));
-          M[r][c] = v;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-#pragma unroll
-      for (int c = r; c < 6; ++c) {
-        double v;
-        if (c == 4) {
-          v = M[r][4];
-        } else {
-          const int gc = (c == 5) ? 4 : c;
-          v = M[r][0] * (double)Pg[5 * gc];
-#pragma unroll
-          for (int k = 1; k < 5; ++k) v += M[r][k] * (double)Pg[5 * gc + k];
-          if (c == 5) v += M[r][5];
-        }
-        Cs[ut(r, c)] = v;
-      }
-    }
-  }
-  const PlaneD &pl = planes[L.firstPlane];
-  stepperUpdate(L, pl, xs, Cs, P.mass);
-  if (!P.faithful) planeJacToGlobal(L, pl);
-  L.navDir = -1;
-  ssInit(L, -1. * DBL_MAX);
-  L.pathAcc = 0.;
-  return true;
-}
-
-// ---------------------------------------------------------------------------
 // The general gain-matrix smoother (GainMatrixSmoother.hpp:21-94) for fits
 // with material noise, where the closed forms above do not hold:
 //   G = C_f J^T C_p'^-1,  x_s = x_f + G (x_s' - x_p'),
@@ -2006,10 +1862,12 @@ static __device__ __forceinline__ bool smoothNoise(const Params &P, int64_t u, i
   return true;
 }
 
+// Actor::finalize (KalmanFitter.hpp:360-393); false on a NaN gain.  Only fits
+// with material reach it: the adjoint runs its own smoother.
 template <typename R, typename H>
 __device__ bool finalizeSmooth(Lane<R, H> &L, const Params &P, const PlaneD *planes) {
   L.smoothed = true;
-  if (H::kMaterial && P.materialEffects) {
+  if constexpr (H::kMaterial) {
     double xs[6], Cs[21];
     if (!smoothNoise(P, L.wsIdx, L.idx, L.measStates, xs, Cs)) return false;
     const PlaneD &pl = planes[L.firstPlane];
@@ -2018,104 +1876,7 @@ __device__ bool finalizeSmooth(Lane<R, H> &L, const Params &P, const PlaneD *pla
     L.navDir = -1;
     ssInit(L, -1. * DBL_MAX);
     L.pathAcc = 0.;
-    return true;
   }
-  if (!P.oSmoothed) return finalizeSmoothGain<R>(L, P, planes);
-  const int n = L.measStates;
-  double xs[6], Cs[21];
-#pragma unroll
-  for (int e = 0; e < 6; ++e) xs[e] = *wsPtr(P, L, n - 1, 6 + e);
-  // the stepper holds the last filtered covariance
-#pragma unroll
-  for (int e = 0; e < 21; ++e) Cs[e] = L.cov(e);
-  if (P.oSmoothed) {
-#pragma unroll
-    for (int e = 0; e < 6; ++e)
-      P.oSmoothed[((size_t)(n - 1) * 27 + e) * P.stride + L.idx] = xs[e];
-#pragma unroll
-    for (int e = 0; e < 21; ++e)
-      P.oSmoothed[((size_t)(n - 1) * 27 + 6 + e) * P.stride + L.idx] = Cs[e];
-  }
-  for (int i = n - 2; i >= 0; --i) {
-    double xp[6], Jn[25], xf[6], G[25];
-#pragma unroll
-    for (int e = 0; e < 6; ++e) xp[e] = *wsPtr(P, L, i + 1, e);
-#pragma unroll
-    for (int e = 0; e < 25; ++e) Jn[e] = *wsPtr(P, L, i + 1, 12 + e);
-#pragma unroll
-    for (int e = 0; e < 6; ++e) xf[e] = *wsPtr(P, L, i, 6 + e);
-    invJacobian(Jn, G);
-    bool nan = false;
-#pragma unroll
-    for (int e = 0; e < 25; ++e) nan = nan || (G[e] != G[e]);
-    if (nan) return false;
-    double dx[6];
-#pragma unroll
-    for (int e = 0; e < 6; ++e) dx[e] = xs[e] - xp[e];
-    // rows 0..3 and 5 of G have columns 0..4 stored; row 4 = e4, G(5,5) = 1
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      if (r == 4) {
-        xs[4] = xf[4] + dx[4];
-      } else {
-        const int gr = (r == 5) ? 4 : r;
-        double g = G[5 * gr] * dx[0];
-#pragma unroll
-        for (int k = 1; k < 5; ++k) g += G[5 * gr + k] * dx[k];
-        if (r == 5) g += dx[5];
-        xs[r] = xf[r] + g;
-      }
-    }
-    // Cs <- G Cs G^T
-    double M[6][6];
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        if (r == 4) {
-          M[r][c] = Cs[sidx(4, c)];
-        } else {
-          const int gr = (r == 5) ? 4 : r;
-          double v = G[5 * gr] * Cs[sidx(0, c)];
-#pragma unroll
-          for (int k = 1; k < 5; ++k) v += G[5 * gr + k] * Cs[sidx(k, c)];
-          if (r == 5) v += Cs[sidx(5, c)];
-          M[r][c] = v;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 6; ++r) {
-#pragma unroll
-      for (int c = r; c < 6; ++c) {
-        double v;
-        if (c == 4) {
-          v = M[r][4];
-        } else {
-          const int gc = (c == 5) ? 4 : c;
-          v = M[r][0] * G[5 * gc];
-#pragma unroll
-          for (int k = 1; k < 5; ++k) v += M[r][k] * G[5 * gc + k];
-          if (c == 5) v += M[r][5];
-        }
-        Cs[ut(r, c)] = v;
-      }
-    }
-    if (P.oSmoothed) {
-#pragma unroll
-      for (int e = 0; e < 6; ++e)
-        P.oSmoothed[((size_t)i * 27 + e) * P.stride + L.idx] = xs[e];
-#pragma unroll
-      for (int e = 0; e < 21; ++e)
-        P.oSmoothed[((size_t)i * 27 + 6 + e) * P.stride + L.idx] = Cs[e];
-    }
-  }
-  const PlaneD &pl = planes[L.firstPlane];
-  stepperUpdate(L, pl, xs, Cs, P.mass);
-  if (!P.faithful) planeJacToGlobal(L, pl);
-  L.navDir = -1;
-  ssInit(L, -1. * DBL_MAX);
-  L.pathAcc = 0.;
   return true;
 }
 
@@ -2146,8 +1907,8 @@ __device__ __forceinline__ int updateSurfaceStatus(Lane<R, H> &L, const Params &
   return kMissed;
 }
 
-template <typename R, typename H>
-__device__ __forceinline__ void navStatus(Lane<R, H> &L, const Params &P, const PlaneD *planes) {
+template <class LT>
+__device__ __forceinline__ void navStatus(LT &L, const Params &P, const PlaneD *planes) {
   L.current = -1;
   L.navCache = -1;
   if (L.next != L.nSeq) {
@@ -2167,8 +1928,8 @@ __device__ __forceinline__ void navStatus(Lane<R, H> &L, const Params &P, const 
   }
 }
 
-template <typename R, typename H>
-__device__ __forceinline__ void navTarget(Lane<R, H> &L, const Params &P, const PlaneD *planes) {
+template <class LT>
+__device__ __forceinline__ void navTarget(LT &L, const Params &P, const PlaneD *planes) {
   L.current = -1;
   if (L.next != L.nSeq) {
     // the repeated intersection would set the same step constraint again
@@ -2275,7 +2036,7 @@ template <typename R, typename H> __device__ __forceinline__ bool aborters(Lane<
   return limit;
 }
 
-template <typename R, typename H> __device__ __forceinline__ void finish(Lane<R, H> &L, const Params &P) {
+template <class LT> __device__ __forceinline__ void finish(LT &L, const Params &P) {
   int st;
   if (!L.result)
     st = L.smoothed ? KF_TRACK_SMOOTHER_NAN : KF_TRACK_MEAS_MISMATCH;
@@ -2296,7 +2057,7 @@ template <typename R, typename H> __device__ __forceinline__ void finish(Lane<R,
 // (heavy actor work) is due, or the track is done; runEvent() executes the
 // pending actor call with heavy work allowed and continues.
 // ---------------------------------------------------------------------------
-template <typename R, typename H> __device__ void advance(Lane<R, H> &L, const Params &P, const PlaneD *planes) {
+template <class LT> __device__ void advance(LT &L, const Params &P, const PlaneD *planes) {
   for (;;) {
     switch (L.pc) {
     case PC_PRE:
