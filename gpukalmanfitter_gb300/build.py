@@ -23,7 +23,7 @@ LIB = LIBDIR / "libgb300kf.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # fit kernels: one file per precision and register budget
 CU_SOURCES = ["kf_capi.cu", "kf_launch.cu", "kf_batch.cu", "kf_fit_material.cu",
-              "kf_fit_material_states.cu", "kf_diag.cu", "kf_noalloc.cu", "kf_adjoint.cu",
+              "kf_fit_material_states.cu", "kf_fit_fp64_any.cu", "kf_diag.cu", "kf_noalloc.cu", "kf_adjoint.cu",
               "kf_sim.cu"] + [f"kf_fit_{p}_{r}.cu" for p in ("fp64", "mixed")
                               for r in (255, 168, 128, 96)]
 CXX_SOURCES = ["synth.cpp", "kf_io.cpp", "kf_fieldmap.cpp"]
@@ -56,7 +56,7 @@ def _stale(target: Path, deps: list[Path]) -> bool:
 def _run(cmd: list[str]) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError(f"build step failed: {' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
+        raise RuntimeError(f"build step failed: {' '.join(cmd)}\n{res.stdout[-4000:]}\n{res.stderr[-4000:]}")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

@@ -130,6 +130,10 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
   P.tolLoF = (float)(P.tol * 0.99);
   // below the reference's floor of the error estimate (1e-20) FP64 decides
   P.tolAcceptF = P.tol > 1e-19 ? (float)(P.tol * (1. - 1e-5)) : -1.f;
+  // |A d + y A^2 d|_1 <= sqrt(3) (1 + |y|) |d|, |y| <= 0.1: err <= 0.4764 |h y x|
+  const double bound = P.tol > 1e-19 ? P.tol / 0.477 : -1.;
+  P.errBound = bound < 0. ? -1 : 0;
+  if (bound > 0.) std::memcpy(&P.errBound, &bound, sizeof(bound));
   for (int k = 0; k < in->n_surfaces; ++k) {
     PlaneD &pl = P.planes[k];
     for (int r = 0; r < 3; ++r) {
@@ -138,6 +142,7 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
       pl.V[r] = geo->rotation[9 * k + 3 * r + 1];
       pl.T[r] = geo->rotation[9 * k + 3 * r + 2];
     }
+    pl.tc = pl.T[0] * pl.c[0] + pl.T[1] * pl.c[1] + pl.T[2] * pl.c[2];
     {
       double m[6] = {0., 0., 0., 0., 0., 0.};
       if (geo->material)

@@ -54,6 +54,7 @@ constexpr int kStateStride = 37; // doubles per stored measurement state
 
 struct PlaneD {
   double c[3], U[3], V[3], T[3];
+  double tc; // T . c
 };
 
 struct FieldD {
@@ -73,7 +74,8 @@ struct Params {
   int maxSteps, maxTrials, smoothing, faithful;
   double tol, cutoff, mass, overstep, surfTol, outlierCut;
   float tolLoF;         // mixed form: FP32 error estimates up to this accept
-  float tolAcceptF;     // FP64 forms: FP32-rounded error estimates up to this accept
+  float tolAcceptF;     // FP64 map form: FP32-rounded error estimates up to this accept
+  long long errBound;   // FP64 uniform form: |h y x| up to this (bits of a double) accept
   const double *meas;
   const uint64_t *mask;
   const int32_t *nplanes;
@@ -89,7 +91,6 @@ struct Params {
   // FP64 fit in a uniform field: the field along z of the frame that the
   // planes are given in (rot: its axes, rows; the identity unless rotated)
   double Bz, rot[9];
-  float rotf[9];
   int rotated;
   FieldD field;
   PlaneD planes[KF_MAX_PLANES];

@@ -52,7 +52,11 @@
 
 namespace kfd {
 
-enum FitForm { kUniform64 = 0, kGrid64 = 1, kMixed = 2 };
+// kUniform64: FP64, uniform field along +-z; kUniformAny: in any other
+// direction (planes rotated into the field's frame); kGrid64: FP64, field
+// map; kMixed: mixed precision, any field
+enum FitForm { kUniform64 = 0, kGrid64 = 1, kMixed = 2, kUniformAny = 3 };
+__host__ __device__ constexpr bool isUniform(int form) { return form == kUniform64 || form == kUniformAny; }
 
 // ---- FP64 reciprocal and reciprocal square root -----------------------------
 // The hardware's 20-bit estimate and one third-order step (Halley's family):
@@ -97,6 +101,7 @@ template <> struct LegState<kUniform64> {
   double g, b, r, q1, s, c[2], a[2];
   double y, dx, dy; // last step: h q/p B and the direction it started from (k4)
 };
+template <> struct LegState<kUniformAny> : LegState<kUniform64> {};
 // field map: columns phi, theta, q/p of position and direction
 template <> struct LegState<kGrid64> {
   double p[3][3], v[3][3], s, k4[3];
@@ -116,6 +121,7 @@ struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
   static constexpr bool kMat = MAT_;
   double pos[3], dir[3]; // FP64 uniform field: in the field's frame
   double q, qop, t, dtds, d37;
+  double idn;            // 1 / (T . dir) of the plane last looked at
   double ss[4];
   int ssDir, navDir;
   LegState<FORM> g;
@@ -168,7 +174,7 @@ __device__ __forceinline__ Trig trigOf(const double d[3], double &invS) {
 // global <-> field frame (the identity unless the field is off the z axis)
 template <class LT>
 __device__ __forceinline__ void toGlobal(const Params &P, const double v[3], double o[3]) {
-  if (LT::kForm == kUniform64 && P.rotated) {
+  if (LT::kForm == kUniformAny) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) o[i] = P.rot[i] * v[0] + P.rot[3 + i] * v[1] + P.rot[6 + i] * v[2];
   } else {
@@ -178,7 +184,7 @@ __device__ __forceinline__ void toGlobal(const Params &P, const double v[3], dou
 }
 template <class LT>
 __device__ __forceinline__ void toFrame(const Params &P, const double v[3], double o[3]) {
-  if (LT::kForm == kUniform64 && P.rotated) {
+  if (LT::kForm == kUniformAny) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       o[i] = P.rot[3 * i] * v[0] + P.rot[3 * i + 1] * v[1] + P.rot[3 * i + 2] * v[2];
@@ -211,7 +217,7 @@ __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, b
 template <int FORM, bool MAT>
 __device__ __forceinline__ void legReset(FitLane<FORM, MAT> &L, const Trig &t) {
   L.stepped = false;
-  if constexpr (FORM == kUniform64) {
+  if constexpr (isUniform(FORM)) {
     L.g.g = 1.;
     L.g.b = L.g.r = L.g.q1 = L.g.s = 0.;
     L.g.c[0] = L.g.c[1] = L.g.a[0] = L.g.a[1] = 0.;
@@ -268,92 +274,86 @@ __device__ __forceinline__ bool rejectTrial(LT &L, const Params &P, double err, 
 //   al = y (1 - x/6), be = x (1/2 - x/24), mu = h y (1/2 - x/24), nu = h x/6,
 // the same two matrices D_B, D_A for the transport Jacobian, and the q/p
 // column's sources are their q/p derivatives (kfa::polyAcceptFwd has the
-// general field).  |dir'|^2 - |dir|^2 = |dir_perp|^2 x^3 (x/576 - 1/72), so
-// that the normalisation is a product with 1 - half of that (FP32 suffices
-// where it is below 1e-10).  The error estimate
+// general field).  The error estimate
 // h^2 |k1 - k2 - k3 + k4|_1 = |h y| x/4 |A dir + y A^2 dir|_1
-// decides in FP32 unless it lies within 1e-5 of the tolerance or above (the
-// FP32 value is good to 1e-6).
-template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kUniform64, MAT> &L, const Params &P) {
+// is at most |h y| x times P.errBound's factor for |y| <= 0.1, which accepts
+// with one product; only beyond that bound it is evaluated.
+// |dir'|^2 - |dir|^2 = |dir_perp|^2 x^3 (x/576 - 1/72): below half an ulp, so
+// that there is nothing to normalise, where |x| < 1e-5.
+template <int FORM, bool MAT>
+__device__ __forceinline__ void stepUniform(FitLane<FORM, MAT> &L, const Params &P) {
   long nTrials = 0;
   double h = ssValue(L);
   const double k = L.qop * P.Bz;
   const double dx = L.dir[0], dy = L.dir[1];
-  const float kf = (float)k, dxf = (float)dx, dyf = (float)dy;
+  double y, x, hy;
   for (;;) {
     L.rkTrials++;
-    {
-      const float hf = (float)h, yf = hf * kf;
-      const float v0 = dyf - yf * dxf, v1 = -dxf - yf * dyf;
-      float n1;
-      if (P.rotated)
-        n1 = fabsf(P.rotf[0] * v0 + P.rotf[3] * v1) + fabsf(P.rotf[1] * v0 + P.rotf[4] * v1) +
-             fabsf(P.rotf[2] * v0 + P.rotf[5] * v1);
-      else
-        n1 = fabsf(v0) + fabsf(v1);
-      if (0.25f * fabsf(hf * yf) * (yf * yf) * n1 <= P.tolAcceptF) break;
-    }
-    const double y = h * k;
+    y = h * k;
+    x = y * y;
+    hy = h * y;
+    if (akey(hy * x) <= P.errBound && akey(y) <= 0x3fb999999999999aLL) break;
     const double v0 = fma(-y, dx, dy), v1 = fma(-y, dy, -dx);
     double n1;
-    if (P.rotated)
+    if (FORM == kUniformAny)
       n1 = fabs(P.rot[0] * v0 + P.rot[3] * v1) + fabs(P.rot[1] * v0 + P.rot[4] * v1) +
            fabs(P.rot[2] * v0 + P.rot[5] * v1);
     else
       n1 = fabs(v0) + fabs(v1);
-    const double e0 = 0.25 * fabs(h * y) * (y * y) * n1;
+    const double e0 = 0.25 * fabs(hy) * x * n1;
     const double err = e0 < 1e-20 ? 1e-20 : e0;
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) return;
   }
   auto &g = L.g;
-  const double y = h * k, x = y * y;
   const double m = fma(x, -1. / 24., 0.5), n = fma(x, -1. / 6., 1.);
   const double al = y * n, be1 = fma(-x, m, 1.);
-  const double mu = h * y * m, nu = h * x * (1. / 6.), hn = h - nu;
-  // q/p derivatives: of y h B, ...
+  const double mu = hy * m, nu = h * x * (1. / 6.), hn = h - nu;
+  // q/p derivatives (y's is h B)
   const double hb = h * P.Bz, hhb = h * hb;
   const double al1 = hb * fma(x, -0.5, 1.), be2 = hb * al;
   const double mu1 = hhb * fma(x, -0.125, 0.5), nu1 = hhb * y * (1. / 3.);
   // q/p column
-  const double a0 = g.a[0] + hn * g.c[0] + mu * g.c[1] + mu1 * dy - nu1 * dx;
-  const double a1 = g.a[1] + hn * g.c[1] - mu * g.c[0] - mu1 * dx - nu1 * dy;
-  const double c0 = be1 * g.c[0] + al * g.c[1] + al1 * dy - be2 * dx;
-  const double c1 = be1 * g.c[1] - al * g.c[0] - al1 * dx - be2 * dy;
+  const double a0 = fma(hn, g.c[0], fma(mu, g.c[1], fma(mu1, dy, fma(-nu1, dx, g.a[0]))));
+  const double a1 = fma(hn, g.c[1], fma(-mu, g.c[0], fma(-mu1, dx, fma(-nu1, dy, g.a[1]))));
+  const double c0 = fma(be1, g.c[0], fma(al, g.c[1], fma(al1, dy, -be2 * dx)));
+  const double c1 = fma(be1, g.c[1], fma(-al, g.c[0], fma(-al1, dx, -be2 * dy)));
   g.a[0] = a0;
   g.a[1] = a1;
   g.c[0] = c0;
   g.c[1] = c1;
   // transport of the direction columns
-  g.r += hn * g.g - mu * g.b;
-  g.q1 += hn * g.b + mu * g.g;
+  g.r = fma(hn, g.g, fma(-mu, g.b, g.r));
+  g.q1 = fma(hn, g.b, fma(mu, g.g, g.q1));
   g.s += h;
-  const double gg = be1 * g.g - al * g.b;
-  g.b = be1 * g.b + al * g.g;
+  const double gg = fma(be1, g.g, -al * g.b);
+  g.b = fma(be1, g.b, al * g.g);
   g.g = gg;
   g.y = y;
   g.dx = dx;
   g.dy = dy;
   // the track
-  L.pos[0] += hn * dx + mu * dy;
-  L.pos[1] += hn * dy - mu * dx;
-  L.pos[2] += h * L.dir[2];
-  double ndx = be1 * dx + al * dy, ndy = be1 * dy - al * dx, ndz = L.dir[2];
-  const float xf = (float)x, sf = dxf * dxf + dyf * dyf;
-  const float eps = sf * (xf * xf * xf) * (xf * (1.f / 576.f) - (1.f / 72.f));
-  if (fabsf(eps) <= 1e-10f) {
-    const double f1 = (double)(-0.5f * eps);
-    L.dir[0] = fma(ndx, f1, ndx);
-    L.dir[1] = fma(ndy, f1, ndy);
-    L.dir[2] = fma(ndz, f1, ndz);
-  } else {
-    const double in = rsqrt(ndx * ndx + ndy * ndy + ndz * ndz);
-    L.dir[0] = ndx * in;
-    L.dir[1] = ndy * in;
-    L.dir[2] = ndz * in;
+  L.pos[0] = fma(hn, dx, fma(mu, dy, L.pos[0]));
+  L.pos[1] = fma(hn, dy, fma(-mu, dx, L.pos[1]));
+  L.pos[2] = fma(h, L.dir[2], L.pos[2]);
+  L.dir[0] = fma(be1, dx, al * dy);
+  L.dir[1] = fma(be1, dy, -al * dx);
+  if (!(akey(x) < 0x3ee4f8b588e368f1LL)) { // |x| >= 1e-5
+    const double n2 = L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1] + L.dir[2] * L.dir[2];
+    double f = fma(n2, -0.5, 1.5);
+    if (fabs(n2 - 1.) > 1e-9) f = rsqrt(n2); // large turning steps
+    L.dir[0] *= f;
+    L.dir[1] *= f;
+    L.dir[2] *= f;
   }
   L.stepped = true;
   L.rkSteps++;
+}
+template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kUniform64, MAT> &L, const Params &P) {
+  stepUniform(L, P);
+}
+template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kUniformAny, MAT> &L, const Params &P) {
+  stepUniform(L, P);
 }
 
 // an FP32 value as FP64 on the integer pipe (normal values exactly; FP32
@@ -585,9 +585,9 @@ __device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT> &L, const 
   const double denom = pl.T[0] * L.dir[0] + pl.T[1] * L.dir[1] + pl.T[2] * L.dir[2];
   if (denom != 0.0) {
     // along dir; the reference's path is along navDir * dir
-    const double along = (pl.T[0] * (pl.c[0] - L.pos[0]) + pl.T[1] * (pl.c[1] - L.pos[1]) +
-                          pl.T[2] * (pl.c[2] - L.pos[2])) *
-                         rcpFast(denom);
+    L.idn = rcpFast(denom);
+    const double along =
+        fma(-pl.T[0], L.pos[0], fma(-pl.T[1], L.pos[1], fma(-pl.T[2], L.pos[2], pl.tc))) * L.idn;
     if (akey(along) < akey(P.surfTol)) {
       ssRelease(L, kActor);
       return kOnSurface;
@@ -657,10 +657,11 @@ __device__ __forceinline__ void lastAxes(const LT &L, const Params &P, const Pla
 // 3: theta, 4: q/p.  At the start, a shift in phi also moves the point at
 // distance loc0 from the line (initJacobianToGlobal, LineSurface.ipp:63-112):
 // by -loc0 (cos phi, sin phi, 0); loc0 is `o`.
-template <bool MAT>
-__device__ __forceinline__ void legColumn(const FitLane<kUniform64, MAT> &L, const Params &P,
-                                          const Trig &t, double o, int c, double p[3], double v[3]) {
-  using LT = FitLane<kUniform64, MAT>;
+template <int FORM, bool MAT>
+__device__ __forceinline__ typename std::enable_if<isUniform(FORM)>::type
+legColumn(const FitLane<FORM, MAT> &L, const Params &P, const Trig &t, double o, int c, double p[3],
+          double v[3]) {
+  using LT = FitLane<FORM, MAT>;
   const auto &g = L.g;
   if (c == 4) {
     p[0] = g.a[0];
@@ -678,11 +679,11 @@ __device__ __forceinline__ void legColumn(const FitLane<kUniform64, MAT> &L, con
     const double ge[3] = {t.cT * t.cP, t.cT * t.sP, -t.sT};
     toFrame<LT>(P, ge, e);
   }
-  p[0] = g.r * e[0] + g.q1 * e[1];
-  p[1] = g.r * e[1] - g.q1 * e[0];
+  p[0] = fma(g.r, e[0], g.q1 * e[1]);
+  p[1] = fma(g.r, e[1], -g.q1 * e[0]);
   p[2] = g.s * e[2];
-  v[0] = g.g * e[0] + g.b * e[1];
-  v[1] = g.g * e[1] - g.b * e[0];
+  v[0] = fma(g.g, e[0], g.b * e[1]);
+  v[1] = fma(g.g, e[1], -g.b * e[0]);
   v[2] = e[2];
   if (c == 2 && L.measStates == 0) {
     const double go[3] = {-o * t.cP, -o * t.sP, 0.};
@@ -706,12 +707,13 @@ __device__ __forceinline__ void legColumn(const FitLane<kGrid64, MAT> &L, const 
   }
 }
 // k4 of the last step
-template <bool MAT>
-__device__ __forceinline__ void lastK4(const FitLane<kUniform64, MAT> &L, const Params &P, double k4[3]) {
+template <int FORM, bool MAT>
+__device__ __forceinline__ typename std::enable_if<isUniform(FORM)>::type
+lastK4(const FitLane<FORM, MAT> &L, const Params &P, double k4[3]) {
   const double k = L.qop * P.Bz, y = L.g.y, x = y * y;
   const double w1 = k * fma(x, -0.5, 1.), w2 = k * y * fma(x, -0.25, 1.);
-  k4[0] = w1 * L.g.dy - w2 * L.g.dx;
-  k4[1] = -(w1 * L.g.dx) - w2 * L.g.dy;
+  k4[0] = fma(w1, L.g.dy, -w2 * L.g.dx);
+  k4[1] = fma(-w1, L.g.dx, -w2 * L.g.dy);
   k4[2] = 0.;
 }
 template <bool MAT>
@@ -725,7 +727,12 @@ template <int FORM, bool MAT> __device__ __forceinline__ double legPath(const Fi
 }
 
 __device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
-  return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+  return fma(a[0], b[0], fma(a[1], b[1], a[2] * b[2]));
+}
+// a . b where flat says that the z products vanish (a multiplication by a
+// literal 0 costs an FP64 instruction like any other)
+__device__ __forceinline__ double dotz(bool flat, const double a[3], const double b[3]) {
+  return flat ? fma(a[0], b[0], a[1] * b[1]) : dot3(a, b);
 }
 
 // FP64 forms, at a surface with local axes a0, a1, where a parameter's path
@@ -745,7 +752,10 @@ __device__ __forceinline__ void boundRows(const LT &L, const Params &P, const Pl
     u0 = dot3(a0, L.dir);
     u1 = dot3(a1, L.dir);
   }
-  const double fk0 = dot3(f0, k4), fk1 = dot3(f1, k4);
+  // vectors without a z component: the phi row (but in a turned frame), and in
+  // a uniform field along z the k4 and the phi and q/p columns
+  constexpr bool kFlatRow = LT::kForm != kUniformAny, kFlat = LT::kForm == kUniform64;
+  const double fk0 = dotz(kFlatRow, f0, k4), fk1 = dotz(kFlat, f1, k4);
   const double dt = L.stepped ? L.dtds : 0.;
   double A0[3], A1[3];
   if (!LINE) {
@@ -773,11 +783,12 @@ __device__ __forceinline__ void boundRows(const LT &L, const Params &P, const Pl
   for (int c = 2; c < 5; ++c) {
     double p[3], v[3];
     legColumn(L, P, tl, o, c, p, v);
-    const double s = LINE ? dot3(sp, p) + dot3(sv, v) : dot3(sp, p);
-    J[0][c] = LINE ? fma(-u0, s, dot3(a0, p)) : dot3(A0, p);
-    J[1][c] = LINE ? fma(-u1, s, dot3(a1, p)) : dot3(A1, p);
-    J[2][c] = fma(-fk0, s, dot3(f0, v));
-    J[3][c] = fma(-fk1, s, dot3(f1, v));
+    const bool flat = kFlat && c != 3;
+    const double s = LINE ? dotz(flat, sp, p) + dotz(flat, sv, v) : dotz(flat, sp, p);
+    J[0][c] = LINE ? fma(-u0, s, dotz(flat, a0, p)) : dotz(flat, A0, p);
+    J[1][c] = LINE ? fma(-u1, s, dotz(flat, a1, p)) : dotz(flat, A1, p);
+    J[2][c] = fma(-fk0, s, dotz(kFlatRow, f0, v));
+    J[3][c] = fma(-fk1, s, dotz(flat, f1, v));
     if (time) J5[c] = (c == 4) ? fma(-dt, s, legPath(L) * L.d37) : -dt * s;
   }
 }
@@ -805,9 +816,9 @@ __device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT> &L, const
   const double o = L.measStates == 0 ? P.start[L.idx] : 0.;
   double sp[3] = {0., 0., 0.}, f0[3], f1[3];
   if (L.stepped) {
-    const double id = rcpFast(dot3(pl.T, L.dir));
+    // (the track is on this plane: idn is its)
 #pragma unroll
-    for (int i = 0; i < 3; ++i) sp[i] = pl.T[i] * id;
+    for (int i = 0; i < 3; ++i) sp[i] = pl.T[i] * L.idn;
   }
   angleRows<LT>(P, tr, invS, f0, f1);
   boundRows<false>(L, P, planes, tl, o, pl.U, pl.V, sp, sp, f0, f1, time, J, J5);
@@ -857,9 +868,7 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT> &L, con
     }
   }
   // ---- straight-line part, FP64
-  const double dp = dot3(pl.T, L.dir);
-  const double idp = rcpFast(dp);
-  const double nv[3] = {pl.T[0] * idp, pl.T[1] * idp, pl.T[2] * idp};
+  const double nv[3] = {pl.T[0] * L.idn, pl.T[1] * L.idn, pl.T[2] * L.idn};
 #pragma unroll
   for (int c = 0; c < 4; ++c) s0[c] = nv[0] * P0[0][c] + nv[1] * P0[1][c] + nv[2] * P0[2][c];
   double A0[3], A1[3];
@@ -1737,8 +1746,9 @@ __device__ __forceinline__ void initFit(FitLane<FORM, MAT> &L, const Params &P, 
 
 // ---------------------------------------------------------------------------
 // The Kalman actor (KalmanFitter.hpp:216-273), as kf_device.cuh's: with heavy
-// == false it only runs when no filter update, smoothing or final transport
-// is due, and returns false without touching the state otherwise.
+// == false it only runs between surfaces, where no filter update, smoothing or
+// final transport can be due, and returns false without touching the state
+// otherwise.
 // ---------------------------------------------------------------------------
 template <int FORM, bool MAT>
 __device__ __forceinline__ bool actor(FitLane<FORM, MAT> &L, const Params &P, const PlaneD *planes,
@@ -1746,10 +1756,10 @@ __device__ __forceinline__ bool actor(FitLane<FORM, MAT> &L, const Params &P, co
   const bool onPlane = L.current >= 0 && !L.smoothed && !L.finished;
   const bool hit = onPlane && ((L.mask >> L.current) & 1ull);
   if (!heavy) {
-    const int ms = L.measStates + (hit ? 1 : 0);
-    const bool fin = (ms == L.nHits || (ms > 0 && L.navBreak)) && !L.smoothed && !L.finished &&
-                     P.smoothing;
-    if (hit || fin) return false;
+    // every plane, hit or not, is a meeting point of the warp (see fitWarp)
+    const bool fin = (L.measStates == L.nHits || (L.measStates > 0 && L.navBreak)) && !L.smoothed &&
+                     !L.finished && P.smoothing;
+    if (onPlane || fin) return false;
     if (L.smoothed && !L.finished) {
       if (L.targetReached || L.current == -2) return false;
       double u;

@@ -6,10 +6,13 @@
 // fit them and claim again until the queue is empty; without (kf_fit_batch),
 // warp w fits tracks 32 w ... 32 w + 31.
 //
-// Lanes step independently and park at heavy actor work (filter update,
-// smoothing, final transport); when every lane of the warp is parked or done,
-// the parked lanes run their events together, so the FP64-heavy Kalman
-// algebra executes without divergence.
+// Lanes step independently and park at every plane they reach and at other
+// heavy actor work (smoothing, final transport); when every lane of the warp
+// is parked or done, the parked lanes run their events together, so the
+// FP64-heavy Kalman algebra executes without divergence.  A lane whose plane
+// has no hit waits too: passing it would put that lane a plane ahead, and its
+// steps there would run with the others idle (tracks with 10 % holes: 1.24
+// instead of 1.45 times the warp instructions of a track without divergence).
 //
 // The block size is a run-time value: an instantiation is a register budget,
 // so that every shape of one budget, queue or not, gives the same bits.

@@ -12,6 +12,8 @@ KF_DECLARE_BUDGET(255)
 KF_DECLARE_BUDGET(168)
 KF_DECLARE_BUDGET(128)
 KF_DECLARE_BUDGET(96)
+KF_DECLARE(launchFit_fp64_any)
+KF_DECLARE(launchFitMaterial_fp64_any)
 KF_DECLARE(launchFitMaterial_fp64_uniform)
 KF_DECLARE(launchFitMaterial_fp64_grid)
 KF_DECLARE(launchFitMaterial_mixed)
@@ -22,13 +24,14 @@ namespace {
 
 using Launch = cudaError_t (*)(const Params &, int, cudaStream_t);
 struct Budget {
-  Launch uniform, grid, mixed;
+  Launch uniform, grid, mixed, anyField; // anyField: a uniform field off the z axis
 };
-#define KF_BUDGET(R) {launchFit_fp64_uniform_##R, launchFit_fp64_grid_##R, launchFit_mixed_##R}
+#define KF_BUDGET(R) \
+  {launchFit_fp64_uniform_##R, launchFit_fp64_grid_##R, launchFit_mixed_##R, launchFit_fp64_any}
 const Budget kBudget255 = KF_BUDGET(255), kBudget168 = KF_BUDGET(168), kBudget128 = KF_BUDGET(128),
              kBudget96 = KF_BUDGET(96);
 const Budget kMaterial = {launchFitMaterial_fp64_uniform, launchFitMaterial_fp64_grid,
-                          launchFitMaterial_mixed};
+                          launchFitMaterial_mixed, launchFitMaterial_fp64_any};
 
 struct Shape {
   int bs, minb;
@@ -87,7 +90,6 @@ static void toFieldFrame(Params &P) {
     P.rot[3 + i] = y[i];
     P.rot[6 + i] = z[i];
   }
-  for (int i = 0; i < 9; ++i) P.rotf[i] = (float)P.rot[i];
   P.Bz = n;
   auto turn = [&](double v[3]) {
     double o[3];
@@ -99,7 +101,7 @@ static void toFieldFrame(Params &P) {
     turn(P.planes[k].c);
     turn(P.planes[k].U);
     turn(P.planes[k].V);
-    turn(P.planes[k].T);
+    turn(P.planes[k].T); // (T . c is unchanged)
   }
 }
 
@@ -115,7 +117,7 @@ cudaError_t launchFit(Params &P, int precision, int bs, int minb, cudaStream_t s
   if (mixed) return b->mixed(P, block, s);
   if (P.field.kind != KF_FIELD_CONSTANT) return b->grid(P, block, s);
   toFieldFrame(P);
-  return b->uniform(P, block, s);
+  return (P.rotated ? b->anyField : b->uniform)(P, block, s);
 }
 
 } // namespace kfh
