@@ -869,7 +869,8 @@ int32_t kf_adjoint_batch(const kf_inputs_t *in, kf_adjoint_outputs_t *out, const
   A.grad = compute_gradient != 0;
   rc = sortQueue(P, reinterpret_cast<int32_t *>(base + L.hist),
                  reinterpret_cast<int32_t *>(base + L.offs),
-                 reinterpret_cast<int32_t *>(base + L.perm), s);
+                 reinterpret_cast<int32_t *>(base + L.perm),
+                 nullptr, s);
   if (rc) return rc;
   const unsigned grid = (unsigned)((n + kLaneSlots - 1) / kLaneSlots);
   adjointKernel<<<grid, kLaneSlots, coldStateBytes<double>(), s>>>(P, A);

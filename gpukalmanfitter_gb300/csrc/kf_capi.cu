@@ -205,8 +205,13 @@ int32_t kf_fit_batch(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t
   Params P;
   fillParams(P, in, out, cfg, geo, field, workspace);
   if (P.n == 0) return KF_SUCCESS;
-  const cudaError_t e = launchFit(P, cfg->precision, 0, 0, static_cast<cudaStream_t>(stream));
-  return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
+  // the work queue in the last two words of the first state's record, which
+  // the fit leaves alone (kf_fit.cuh); launchFit sorts no batch so small that
+  // it does not fit
+  int32_t *w = reinterpret_cast<int32_t *>(static_cast<double *>(workspace) + 35 * P.wsStride);
+  int32_t *v = reinterpret_cast<int32_t *>(static_cast<double *>(workspace) + 36 * P.wsStride);
+  const QueueBuffers q = {w, v, v + kSortBuckets, v + 2 * kSortBuckets};
+  return launchFit(P, cfg->precision, 0, 0, q, static_cast<cudaStream_t>(stream));
 }
 
 // ---- host-buffer convenience ----------------------------------------------

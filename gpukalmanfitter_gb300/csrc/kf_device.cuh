@@ -86,8 +86,9 @@ struct Params {
   int materialEffects;   // kf_config_t.material_effects when the geometry has material
   double *wsCov;         // with material: [S][42][wsStride] predicted and filtered
                          // covariance per state (the general smoother's input)
-  const int32_t *perm;   // batched form: queue position -> track index
-  int32_t *queueCounter; // batched form: next unclaimed queue position
+  const int32_t *perm;   // queue position -> track index (null: the identity)
+  int32_t *queueCounter; // next unclaimed queue position (null: warp w takes the w-th share)
+  int lanes;             // tracks per warp
   // FP64 fit in a uniform field: the field along z of the frame that the
   // planes are given in (rot: its axes, rows; the identity unless rotated)
   double Bz, rot[9];

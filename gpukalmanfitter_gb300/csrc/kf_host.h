@@ -36,15 +36,20 @@ int32_t checkCommon(const kf_inputs_t *in, const kf_config_t *cfg, const kf_geom
 // and most curved first; hist and offs hold kSortBuckets ints each
 constexpr int kSortBuckets = 2048;
 int32_t sortQueue(const kfd::Params &P, int32_t *hist, int32_t *offs, int32_t *perm,
-                  cudaStream_t s);
+                  int32_t *counter, cudaStream_t s);
+// device memory for it: perm of n, hist and offs of kSortBuckets ints, one counter
+struct QueueBuffers {
+  int32_t *perm, *hist, *offs, *counter;
+};
 // compiled launch shapes (threads per block, blocks per SM) of the batched
 // form: the index-th (the first is the default); whether a request (0: the
 // default) is one of them
 bool fitShape(int index, int *bs, int *minb);
 bool shapeCompiled(int bs, int minb);
-// enqueue the fit kernel for P (with a queue: P.queueCounter and P.perm set)
-// on s; the shape applies with a queue and without material
-cudaError_t launchFit(kfd::Params &P, int precision, int bs, int minb, cudaStream_t s);
+// enqueue the fit of P on s: sort and fit kernel.  The shape (0, 0: chosen
+// here) applies without material.
+int32_t launchFit(kfd::Params &P, int precision, int bs, int minb, const QueueBuffers &q,
+                  cudaStream_t s);
 // kernel parameter block from the ABI structures
 void fillParams(kfd::Params &P, const kf_inputs_t *in, const kf_outputs_t *out,
                 const kf_config_t *cfg, const kf_geometry_t *geo, const kf_field_t *field,

@@ -1,10 +1,9 @@
 // kf_kernels.cuh — fit kernels over the per-track lane (kf_fit.cuh).
 //
-// fitTracks: one thread per track.  With a work queue (P.queueCounter, the
-// batched form) a grid of the device's resident capacity whose warps claim 32
-// consecutive queue positions (tracks sorted longest first) with one atomic,
-// fit them and claim again until the queue is empty; without (kf_fit_batch),
-// warp w fits tracks 32 w ... 32 w + 31.
+// fitTracks: one thread per track, P.lanes tracks per warp.  With a queue
+// counter a grid of the device's resident capacity whose warps claim their
+// next tracks (sorted longest first) with one atomic until the queue is
+// empty; without, warp w fits the w-th share.  launchFit chooses.
 //
 // Lanes step independently and park at every plane they reach and at other
 // heavy actor work (smoothing, final transport); when every lane of the warp
@@ -57,19 +56,21 @@ __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ 
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const bool queue = P.queueCounter != nullptr;
+  const int lanes = P.lanes;
   for (;;) {
     int64_t base;
     if (queue) {
       int b = 0;
-      if (lane == 0) b = atomicAdd(P.queueCounter, 32);
+      if (lane == 0) b = atomicAdd(P.queueCounter, lanes);
       base = (int64_t)__shfl_sync(0xffffffffu, b, 0);
     } else {
-      base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+      base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes;
     }
     if (base >= P.n) break;
     const int64_t q = base + lane;
-    const int64_t i = (q < P.n) ? (P.perm ? (int64_t)P.perm[q] : q) : -1;
-    fitWarp<FORM, MAT>(P, sp, i, q < P.n ? q : 0);
+    const bool own = lane < lanes && q < P.n;
+    const int64_t i = own ? (P.perm ? (int64_t)P.perm[q] : q) : -1;
+    fitWarp<FORM, MAT>(P, sp, i, own ? q : 0);
     if (!queue) break;
   }
 }
@@ -87,7 +88,8 @@ __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ 
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
                                (int)kfd::fitSmemBytes<MAT>(MAXT, KF_MAX_PLANES));            \
     if (e != cudaSuccess) return e;                                                          \
-    const int64_t need = (P.n + bs - 1) / bs;                                                \
+    const int64_t per_block = (int64_t)(bs / 32) * P.lanes;                                  \
+    const int64_t need = (P.n + per_block - 1) / per_block;                                  \
     int64_t blocks = need;                                                                   \
     if (P.queueCounter) {                                                                    \
       int dev = 0, sms = 0, per = 0;                                                         \

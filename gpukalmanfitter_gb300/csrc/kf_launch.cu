@@ -1,6 +1,8 @@
 // kf_launch.cu — which compiled fit kernel serves a call.
 #include "kf_host.h"
 
+#include <algorithm>
+
 using kfd::Params;
 
 #define KF_DECLARE(NAME) cudaError_t NAME(const Params &, int, cudaStream_t);
@@ -42,7 +44,8 @@ const Shape kShapes[] = {
     {128, 2, &kBudget255}, {64, 4, &kBudget255},  {256, 1, &kBudget255}, {128, 3, &kBudget168},
     {128, 4, &kBudget128}, {64, 8, &kBudget128},  {256, 2, &kBudget128}, {128, 5, &kBudget96},
 };
-constexpr int kPlainBlock = 32;
+// one-warp blocks spread over the SMs most evenly
+constexpr int kDefaultBlock = 32;
 
 } // namespace
 
@@ -105,19 +108,63 @@ static void toFieldFrame(Params &P) {
   }
 }
 
-cudaError_t launchFit(Params &P, int precision, int bs, int minb, cudaStream_t s) {
-  const bool plain = P.queueCounter == nullptr;
+// How a batch is laid over the chip.  One FP64 instruction of a warp costs the
+// same whatever its active lanes, each SM sub-partition starts one every 64
+// cycles, and four warps (one a sub-partition) fill an SM's FP64 pipe.  So a
+// batch first spreads over 4 warps on every SM with as few tracks a warp as
+// that takes (fewer lanes to wait for: 1000 tracks of 10 planes 560 -> 420
+// us), then over 5 ... 8 of them, the kernel's residency; beyond that warps
+// of 32 tracks claim work from the queue.  Sorting (3 small kernels, 15 us)
+// pays from 8 tracks a warp on.
+struct Spread {
+  int lanes;  // tracks per warp
+  bool sort;  // order the tracks by expected work
+  bool queue; // more warps than the chip holds
+};
+static Spread spread(int64_t n, int sms) {
+  if (n > 0x7f000000) return {32, false, false}; // the queue counts in 32 bits
+  const int64_t full = 32 * (int64_t)sms;
+  const int64_t perSm = std::max<int64_t>(4, (n + full - 1) / full);
+  if (perSm > 8) return {32, true, true};
+  const int lanes = (int)((n + sms * perSm - 1) / (sms * perSm));
+  return {lanes, lanes >= 8, false};
+}
+
+int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers &q, cudaStream_t s) {
   const bool mixed = precision == KF_PRECISION_MIXED;
-  const Shape *shape = plain ? &kShapes[0] : findShape(bs, minb);
-  if (!shape) return cudaErrorInvalidValue;
-  if (P.materialEffects && P.oSmoothed)
-    return (mixed ? launchFitMaterialStates_mixed : launchFitMaterialStates_fp64)(P, 0, s);
+  const Shape *shape = findShape(bs, minb);
+  if (!shape) return fail(KF_ERR_UNSUPPORTED, "no fit kernel for this block size / blocks per SM%s");
+  cudaError_t e;
+  P.lanes = 32;
+  if (P.materialEffects && P.oSmoothed) {
+    e = (mixed ? launchFitMaterialStates_mixed : launchFitMaterialStates_fp64)(P, 0, s);
+    return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
+  }
+  int dev = 0, sms = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return cudaFail(e, "device query");
+  const bool asked = (bs || minb) && !P.materialEffects; // a requested shape: always the queue
+  Spread sp = spread(P.n, sms);
+  if (asked) sp = {32, P.n > kSortBuckets, P.n > kSortBuckets};
+  P.lanes = sp.lanes;
+  if (sp.sort) {
+    const int32_t rc = sortQueue(P, q.hist, q.offs, q.perm, q.counter, s);
+    if (rc) return rc;
+    P.perm = q.perm;
+  }
+  if (sp.queue) P.queueCounter = q.counter;
   const Budget *b = P.materialEffects ? &kMaterial : shape->budget;
-  const int block = plain ? kPlainBlock : (P.materialEffects ? kShapes[0].bs : shape->bs);
-  if (mixed) return b->mixed(P, block, s);
-  if (P.field.kind != KF_FIELD_CONSTANT) return b->grid(P, block, s);
-  toFieldFrame(P);
-  return (P.rotated ? b->anyField : b->uniform)(P, block, s);
+  const int block = asked ? shape->bs : kDefaultBlock;
+  if (mixed) {
+    e = b->mixed(P, block, s);
+  } else if (P.field.kind != KF_FIELD_CONSTANT) {
+    e = b->grid(P, block, s);
+  } else {
+    toFieldFrame(P);
+    e = (P.rotated ? b->anyField : b->uniform)(P, block, s);
+  }
+  return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
 }
 
 } // namespace kfh
