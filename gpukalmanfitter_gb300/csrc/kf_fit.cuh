@@ -382,7 +382,7 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
     return;
   }
   int idx[3];
-  double f[3], h[3];
+  double f[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     // the cell's middle rounds to its index: floor by adding 2^52 + 2^51 to
@@ -399,24 +399,19 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
     }
     idx[a] = i;
     f[a] = (gr - fi) + 0.5;
-    h[a] = 0.5 - (gr - fi);
   }
   const size_t nx = F.n[0], nxy = (size_t)F.n[0] * F.n[1];
   const float4 *g = F.grid + ((size_t)idx[2] * nxy + (size_t)idx[1] * nx + idx[0]);
   const float4 v000 = __ldg(g), v100 = __ldg(g + 1), v010 = __ldg(g + nx), v110 = __ldg(g + nx + 1);
   const float4 v001 = __ldg(g + nxy), v101 = __ldg(g + nxy + 1), v011 = __ldg(g + nxy + nx),
                v111 = __ldg(g + nxy + nx + 1);
-  const double gx = h[0], gy = h[1], gz = h[2];
   const double s = F.scale * qop;
   auto tri = [&](float a000, float a100, float a010, float a110, float a001, float a101,
                  float a011, float a111) {
-    const double c00 = widen(a000) * gx + widen(a100) * f[0];
-    const double c10 = widen(a010) * gx + widen(a110) * f[0];
-    const double c01 = widen(a001) * gx + widen(a101) * f[0];
-    const double c11 = widen(a011) * gx + widen(a111) * f[0];
-    const double c0 = c00 * gy + c10 * f[1];
-    const double c1 = c01 * gy + c11 * f[1];
-    return (c0 * gz + c1 * f[2]) * s;
+    auto mix = [](double a, double b, double w) { return fma(w, b - a, a); };
+    const double c0 = mix(mix(widen(a000), widen(a100), f[0]), mix(widen(a010), widen(a110), f[0]), f[1]);
+    const double c1 = mix(mix(widen(a001), widen(a101), f[0]), mix(widen(a011), widen(a111), f[0]), f[1]);
+    return mix(c0, c1, f[2]) * s;
   };
   B[0] = tri(v000.x, v100.x, v010.x, v110.x, v001.x, v101.x, v011.x, v111.x);
   B[1] = tri(v000.y, v100.y, v010.y, v110.y, v001.y, v101.y, v011.y, v111.y);
@@ -1046,6 +1041,42 @@ __device__ __forceinline__ void updateState(LT &L, const Params &P, const PlaneD
   setMomentum(L, P, fabs(qop), time);
 }
 
+// The material interaction at a plane (kfm::interact's formulas for charge
+// +-1), the direction's trigonometry in t, from 1/p: no square roots but
+// those of E and of the new momentum, one logarithm for the energy loss
+// (above beta gamma 10 the density correction's log(beta gamma) joins it) and
+// one for the scattering.  Returns 1/p after the crossing.
+__device__ __forceinline__ double crossMaterial(const kfm::Slab &sl, int flags, double nd, const Trig &t,
+                                                double ip, double m, double &varPhi, double &varTheta,
+                                                double &varQop) {
+  varPhi = varTheta = varQop = 0.;
+  const double pc = rcpFast(fabs(nd)); // path correction
+  const double p = rcpFast(ip), x = m * ip, q2b = fma(x, x, 1.);
+  if (flags & 1) {
+    const double t2 = sl.x0frac * pc * q2b, a = 13.6e-3 * ip;
+    const double f = fma((double)0.038f, log(t2), 1.);
+    varTheta = a * a * t2 * (f * f);
+    varPhi = varTheta * rcpFast(t.sT * t.sT);
+  }
+  if (!(flags & 2)) return ip;
+  const double eps = 0.5 * kfm::kBetheK * sl.Ne * sl.t0 * pc * q2b;
+  const double bg = p * (1. / m), bg2 = bg * bg, g2 = 1. + bg2;
+  const double gamma = g2 * rsqrtFast(g2);
+  const double mf = kfm::kElectronMass / m;
+  // u wmax = (2 m_e)^2 bg^4 / (1 + 2 gamma mf + mf^2)
+  double arg = (4. * kfm::kElectronMass * kfm::kElectronMass) * bg2 *
+               rcpFast(fma(2. * mf, gamma, fma(mf, mf, 1.)));
+  double c = sl.logI + rcpFast(q2b); // + beta^2
+  if (bg < 10.0) arg *= bg2;
+  else c += sl.plasma - 0.5;
+  const double loss = eps * fma(0.5, log(arg), -c);
+  const double k = ip * ip * (4. / kfm::kFwhmOverSigma) * eps;
+  varQop = q2b * (k * k);
+  const double E = m * gamma;
+  if (!(m < E - loss)) return 1. / 0.; // stopped
+  return rsqrtFast(fma(-loss, 2. * E - loss, p * p));
+}
+
 // any of a Jacobian's entries infinite or NaN (the smoother's NaN gain), on
 // the integer pipe
 __device__ __forceinline__ bool anyBad(const double (&J)[4][5]) {
@@ -1350,16 +1381,14 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT> &L, const Params &P
       updateState(L, P, pl, x0 + dl[0], x1 + dl[1], tn, dl[2], dl[3], L.qop + dl[4], false);
     }
     // the material effects after the filtering (KalmanFitter.hpp:344-345)
-    double dg[3], ng[3];
-    toGlobal<FitLane<FORM, MAT>>(P, L.dir, dg);
-    toGlobal<FitLane<FORM, MAT>>(P, pl.T, ng);
-    kfm::Effects fx;
-    if (kfm::interact(P.planeSlab[k], P.materialEffects, ng, dg, rcpFast(fabs(L.qop)), L.q, P.mass,
-                      fx)) {
-      setMomentum(L, P, 1. / fx.p, false);
-      C[u5(2, 2)] = smax(0., C[u5(2, 2)] + fx.varPhi);
-      C[u5(3, 3)] = smax(0., C[u5(3, 3)] + fx.varTheta);
-      C[u5(4, 4)] = smax(0., C[u5(4, 4)] + fx.varQop);
+    if (P.planeSlab[k].valid) {
+      double vPhi, vTheta, vQop;
+      const double ip = crossMaterial(P.planeSlab[k], P.materialEffects, dot3(pl.T, L.dir), tn,
+                                      fabs(L.qop), P.mass, vPhi, vTheta, vQop);
+      setMomentum(L, P, ip, false);
+      C[u5(2, 2)] = smax(0., C[u5(2, 2)] + vPhi);
+      C[u5(3, 3)] = smax(0., C[u5(3, 3)] + vTheta);
+      C[u5(4, 4)] = smax(0., C[u5(4, 4)] + vQop);
     }
 #pragma unroll
     for (int e = 0; e < 15; ++e) L.C(e) = C[e];

@@ -111,9 +111,9 @@ static void toFieldFrame(Params &P) {
 // How a batch is laid over the chip.  One FP64 instruction of a warp costs the
 // same whatever its active lanes, each SM sub-partition starts one every 64
 // cycles, and four warps (one a sub-partition) fill an SM's FP64 pipe.  So a
-// batch first spreads over 4 warps on every SM with as few tracks a warp as
-// that takes (fewer lanes to wait for: 1000 tracks of 10 planes 560 -> 420
-// us), then over 5 ... 8 of them, the kernel's residency; beyond that warps
+// batch first spreads over 3 warps on every SM with as few tracks a warp as
+// that takes (fewer lanes to wait for: 1000 map tracks mixed 1530 -> 1393
+// us), then over 4 ... 8 of them, the kernel's residency; beyond that warps
 // of 32 tracks claim work from the queue.  Sorting (3 small kernels, 15 us)
 // pays from 8 tracks a warp on.
 struct Spread {
@@ -124,7 +124,7 @@ struct Spread {
 static Spread spread(int64_t n, int sms) {
   if (n > 0x7f000000) return {32, false, false}; // the queue counts in 32 bits
   const int64_t full = 32 * (int64_t)sms;
-  const int64_t perSm = std::max<int64_t>(4, (n + full - 1) / full);
+  const int64_t perSm = std::max<int64_t>(3, (n + full - 1) / full);
   if (perSm > 8) return {32, true, true};
   const int lanes = (int)((n + sms * perSm - 1) / (sms * perSm));
   return {lanes, lanes >= 8, false};
