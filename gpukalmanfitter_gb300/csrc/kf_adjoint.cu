@@ -31,6 +31,7 @@
 
 #include <cstring>
 
+#include "kf_adjoint.cuh"
 #include "kf_adjoint_math.h"
 #include "kf_host.h"
 
@@ -49,39 +50,7 @@ __host__ __device__ constexpr int tapeWords(int S) {
   return S * kTapePerState > kTapeSegment ? S * kTapePerState : kTapeSegment;
 }
 constexpr int kSnapWords = 128;    // doubles per lane checkpoint (visitLane writes 115)
-enum { REC_STEP = 1, REC_ACT = 2, REC_HIT = 3 };
 constexpr int kStepFixed = 33;     // pos 3, dir 3, t, p, transport Jacobian 25
-
-struct AdjParams {
-  const int32_t *perm; // [n] queue position -> track
-  double *stateBar;  // [S][37][n] adjoints of predicted, filtered, Jacobian (by position)
-  double *xs;        // [S][6][n] smoothed parameters (by position)
-  int32_t *info;     // [S][n] plane index | outlier << 8 (by position)
-  double *snap;      // [nCk][kSnapWords][n] (by position)
-  double *tape;      // [tapeCap][n] (by position: a warp's lanes at the same tape
-                     // offset touch one contiguous line)
-  int tapeCap;       // tape words per track
-  int fwdTape;       // the forward records the whole track's tape
-  double *alignPart; // [S][6][n] (by track)
-  double *trackFs;   // [n] per-track d chi2 / d field scale (by track)
-  double *chi2;      // [n]
-  int32_t *status;   // [n]
-  double *gradStart; // [6][stride] or null
-  double B0[3];      // field value before scaling
-  int grad;
-};
-
-__device__ __forceinline__ double hdr(int type, int len) { return (double)(type * 65536 + len); }
-
-// a lane's tape: word k at p[k * n]
-struct TapeRef {
-  const double *p;
-  int64_t n;
-  // each word is read once: a streaming load, so that the tape passing
-  // through does not evict the spilled registers and state arrays from L2
-  __device__ __forceinline__ double operator[](int k) const { return __ldcs(p + (int64_t)k * n); }
-  __device__ __forceinline__ TapeRef operator+(int k) const { return {p + (int64_t)k * n, n}; }
-};
 
 struct TapeHook {
   static constexpr bool kMaterial = false;
@@ -664,8 +633,12 @@ __global__ void __launch_bounds__(kLaneSlots, KF_ADJ_MIN_BLOCKS)
   // every lane stays to the end: the lane program and the reverse sweep run
   // warp-synchronously (idle lanes carry no work)
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; // queue position
-  const bool valid = u < P.n;
+  bool valid = u < P.n;
   const int64_t i = valid ? (int64_t)A.perm[u] : 0;                 // track
+  if (A.onlyMarked) { // the tracks that adjointZ left
+    valid = valid && A.status[i] == kLeft;
+    if (!__any_sync(0xffffffffu, valid)) return;
+  }
   ALane L;
   L.hook.tape = A.tape + (valid ? u : 0);
   L.hook.info = A.info + (valid ? u : 0);
@@ -873,6 +846,14 @@ int32_t kf_adjoint_batch(const kf_inputs_t *in, kf_adjoint_outputs_t *out, const
                  nullptr, s);
   if (rc) return rc;
   const unsigned grid = (unsigned)((n + kLaneSlots - 1) / kLaneSlots);
+  // a field along z: adjointZ; this kernel for any other, and for the tracks
+  // whose tape ran over there
+  A.onlyMarked = 0;
+  if (field->value[0] == 0. && field->value[1] == 0.) {
+    const cudaError_t ez = launchAdjointZ(P, A, s);
+    if (ez != cudaSuccess) return cudaFail(ez, "adjoint kernel launch");
+    A.onlyMarked = 1;
+  }
   adjointKernel<<<grid, kLaneSlots, coldStateBytes<double>(), s>>>(P, A);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cudaFail(e, "adjoint kernel launch");

@@ -115,10 +115,11 @@ struct MixedBlocks {
   double sTr;
 };
 
-template <int FORM, bool MAT_>
+template <int FORM, bool MAT_, class H_ = NoHook>
 struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
   static constexpr int kForm = FORM;
   static constexpr bool kMat = MAT_;
+  static constexpr bool kTape = !std::is_same<H_, NoHook>::value; // the adjoint's forward pass
   double pos[3], dir[3]; // FP64 uniform field: in the field's frame
   double q, qop, t, dtds, d37;
   double idn;            // 1 / (T . dir) of the plane last looked at
@@ -134,7 +135,7 @@ struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
   int pc, steps, status, rkSteps, rkTrials;
   double chi2;
   int64_t idx, wsIdx;
-  NoHook hook;
+  H_ hook;
 
   __device__ __forceinline__ double &cold(int e) const {
     return reinterpret_cast<double *>(kfColdSmem)[e * blockDim.x + threadIdx.x];
@@ -214,8 +215,8 @@ __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, b
 // the jacToGlobal in use from here on: bound parameters on plane `plane` (or
 // the start's line), angles at the direction `t` (re-initialised Jacobians,
 // CovarianceEngine.hpp:169-201)
-template <int FORM, bool MAT>
-__device__ __forceinline__ void legReset(FitLane<FORM, MAT> &L, const Trig &t) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void legReset(FitLane<FORM, MAT, H> &L, const Trig &t) {
   L.stepped = false;
   if constexpr (isUniform(FORM)) {
     L.g.g = 1.;
@@ -280,15 +281,17 @@ __device__ __forceinline__ bool rejectTrial(LT &L, const Params &P, double err, 
 // with one product; only beyond that bound it is evaluated.
 // |dir'|^2 - |dir|^2 = |dir_perp|^2 x^3 (x/576 - 1/72): below half an ulp, so
 // that there is nothing to normalise, where |x| < 1e-5.
-template <int FORM, bool MAT>
-__device__ __forceinline__ void stepUniform(FitLane<FORM, MAT> &L, const Params &P) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void stepUniform(FitLane<FORM, MAT, H> &L, const Params &P) {
   long nTrials = 0;
   double h = ssValue(L);
   const double k = L.qop * P.Bz;
   const double dx = L.dir[0], dy = L.dir[1];
   double y, x, hy;
+  L.hook.stepBegin(L);
   for (;;) {
     L.rkTrials++;
+    L.hook.trial(L, h);
     y = h * k;
     x = y * y;
     hy = h * y;
@@ -303,8 +306,12 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT> &L, const Params 
     const double e0 = 0.25 * fabs(hy) * x * n1;
     const double err = e0 < 1e-20 ? 1e-20 : e0;
     if (err <= P.tol) break;
-    if (!rejectTrial(L, P, err, h, nTrials)) return;
+    if (!rejectTrial(L, P, err, h, nTrials)) {
+      L.hook.stepEnd(L, false);
+      return;
+    }
   }
+  L.hook.stepEnd(L, true);
   auto &g = L.g;
   const double m = fma(x, -1. / 24., 0.5), n = fma(x, -1. / 6., 1.);
   const double al = y * n, be1 = fma(-x, m, 1.);
@@ -349,10 +356,10 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT> &L, const Params 
   L.stepped = true;
   L.rkSteps++;
 }
-template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kUniform64, MAT> &L, const Params &P) {
+template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kUniform64, MAT, H> &L, const Params &P) {
   stepUniform(L, P);
 }
-template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kUniformAny, MAT> &L, const Params &P) {
+template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kUniformAny, MAT, H> &L, const Params &P) {
   stepUniform(L, P);
 }
 
@@ -426,7 +433,7 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
 //   v += h/6 (dk1 + 2 (dk2 + dk3) + dk4)
 // which is D J on those columns (D: transportMatrix, EigenStepper.ipp:50-124)
 // without forming D; the q/p column adds each stage's own k_i / (q/p).
-template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kGrid64, MAT> &L, const Params &P) {
+template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGrid64, MAT, H> &L, const Params &P) {
   long nTrials = 0;
   double h = ssValue(L);
   double b1[3], b2[3], b3[3], k1[3], k2[3], k3[3], k4[3], t[3];
@@ -523,7 +530,7 @@ template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kGrid64, MAT>
 // (the RK partition of the path) would drift from the FP64 fit's by ~3e-6,
 // so that a later decision near the tolerance could go the other way (1e-4 of
 // the perigee's resolution on a few tracks in 1e6).
-template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kMixed, MAT> &L, const Params &P) {
+template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMixed, MAT, H> &L, const Params &P) {
   long nTrials = 0;
   double h = ssValue(L);
   const float qopf = (float)L.qop;
@@ -574,9 +581,9 @@ template <bool MAT> __device__ __forceinline__ void rkStep(FitLane<kMixed, MAT> 
 // Navigation: the plane distance with one short division; magnitudes are
 // compared as integers (|path| < tol for the reference's path^2 < tol^2)
 // ---------------------------------------------------------------------------
-template <int FORM, bool MAT>
-__device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT> &L, const Params &P,
-                                                   const PlaneD &pl, int) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT, H> &L, const Params &P,
+                                                   const PlaneD &pl, int k) {
   const double denom = pl.T[0] * L.dir[0] + pl.T[1] * L.dir[1] + pl.T[2] * L.dir[2];
   if (denom != 0.0) {
     // along dir; the reference's path is along navDir * dir
@@ -590,6 +597,7 @@ __device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT> &L, const 
     const double path = L.navDir < 0 ? -along : along;
     if (okey(path) > okey(-P.overstep) && akey(path) < akey(L.ss[kAborter])) {
       ssUpdate(L, along, kActor, true);
+      L.hook.actorSet(L, k);
       return kReachable;
     }
   }
@@ -598,10 +606,10 @@ __device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT> &L, const 
 
 // LineSurface::intersect (LineSurface.ipp:229-262) along navDir * dir with the
 // start's line (axis z)
-template <int FORM, bool MAT>
-__device__ __forceinline__ void lineIntersect(const FitLane<FORM, MAT> &L, const Params &P, double &u,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void lineIntersect(const FitLane<FORM, MAT, H> &L, const Params &P, double &u,
                                               int &status) {
-  using LT = FitLane<FORM, MAT>;
+  using LT = FitLane<FORM, MAT, H>;
   double pg[3], dg[3];
   toGlobal<LT>(P, L.pos, pg);
   toGlobal<LT>(P, L.dir, dg);
@@ -652,11 +660,11 @@ __device__ __forceinline__ void lastAxes(const LT &L, const Params &P, const Pla
 // 3: theta, 4: q/p.  At the start, a shift in phi also moves the point at
 // distance loc0 from the line (initJacobianToGlobal, LineSurface.ipp:63-112):
 // by -loc0 (cos phi, sin phi, 0); loc0 is `o`.
-template <int FORM, bool MAT>
+template <int FORM, bool MAT, class H>
 __device__ __forceinline__ typename std::enable_if<isUniform(FORM)>::type
-legColumn(const FitLane<FORM, MAT> &L, const Params &P, const Trig &t, double o, int c, double p[3],
+legColumn(const FitLane<FORM, MAT, H> &L, const Params &P, const Trig &t, double o, int c, double p[3],
           double v[3]) {
-  using LT = FitLane<FORM, MAT>;
+  using LT = FitLane<FORM, MAT, H>;
   const auto &g = L.g;
   if (c == 4) {
     p[0] = g.a[0];
@@ -688,8 +696,8 @@ legColumn(const FitLane<FORM, MAT> &L, const Params &P, const Trig &t, double o,
     for (int i = 0; i < 3; ++i) p[i] += w[i];
   }
 }
-template <bool MAT>
-__device__ __forceinline__ void legColumn(const FitLane<kGrid64, MAT> &L, const Params &P,
+template <bool MAT, class H>
+__device__ __forceinline__ void legColumn(const FitLane<kGrid64, MAT, H> &L, const Params &P,
                                           const Trig &t, double o, int c, double p[3], double v[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -702,21 +710,21 @@ __device__ __forceinline__ void legColumn(const FitLane<kGrid64, MAT> &L, const 
   }
 }
 // k4 of the last step
-template <int FORM, bool MAT>
+template <int FORM, bool MAT, class H>
 __device__ __forceinline__ typename std::enable_if<isUniform(FORM)>::type
-lastK4(const FitLane<FORM, MAT> &L, const Params &P, double k4[3]) {
+lastK4(const FitLane<FORM, MAT, H> &L, const Params &P, double k4[3]) {
   const double k = L.qop * P.Bz, y = L.g.y, x = y * y;
   const double w1 = k * fma(x, -0.5, 1.), w2 = k * y * fma(x, -0.25, 1.);
   k4[0] = fma(w1, L.g.dy, -w2 * L.g.dx);
   k4[1] = fma(-w1, L.g.dx, -w2 * L.g.dy);
   k4[2] = 0.;
 }
-template <bool MAT>
-__device__ __forceinline__ void lastK4(const FitLane<kGrid64, MAT> &L, const Params &, double k4[3]) {
+template <bool MAT, class H>
+__device__ __forceinline__ void lastK4(const FitLane<kGrid64, MAT, H> &L, const Params &, double k4[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) k4[i] = L.g.k4[i];
 }
-template <int FORM, bool MAT> __device__ __forceinline__ double legPath(const FitLane<FORM, MAT> &L) {
+template <int FORM, bool MAT, class H> __device__ __forceinline__ double legPath(const FitLane<FORM, MAT, H> &L) {
   if constexpr (FORM == kMixed) return L.sTr;
   else return L.g.s;
 }
@@ -799,11 +807,11 @@ __device__ __forceinline__ void angleRows(const Params &P, const Trig &t, double
 }
 
 // at a plane, FP64 forms; tr: trigonometry of the direction there
-template <int FORM, bool MAT>
-__device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT> &L, const Params &P,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
                                               const PlaneD *planes, const PlaneD &pl, bool time,
                                               Trig &tr, double (&J)[4][5], double (&J5)[5]) {
-  using LT = FitLane<FORM, MAT>;
+  using LT = FitLane<FORM, MAT, H>;
   double dg[3], invS;
   toGlobal<LT>(P, L.dir, dg);
   tr = trigOf(dg, invS);
@@ -829,11 +837,11 @@ __device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT> &L, const
 // out accurate to FP32 rounding of those small terms (an FP32 J moves the
 // fitted perigee by up to 3e-6 of its resolution on the 30-plane map
 // telescope, mostly through the angle rows).
-template <bool MAT>
-__device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT> &L, const Params &P,
+template <bool MAT, class H>
+__device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, const Params &P,
                                               const PlaneD *planes, const PlaneD &pl, bool time,
                                               Trig &tr, double (&J)[4][5], double (&J5)[5]) {
-  using LT = FitLane<kMixed, MAT>;
+  using LT = FitLane<kMixed, MAT, H>;
   double invS;
   tr = trigOf(L.dir, invS);
   const Trig tl = trigLoad(L);
@@ -1110,14 +1118,15 @@ __device__ __forceinline__ Gain gain(double S00, double S01, double S11, double 
 // Actor::filter (KalmanFitter.hpp:284-350, GainMatrixUpdater.hpp:34-106) at a
 // plane with a hit
 // ---------------------------------------------------------------------------
-template <int FORM, bool MAT>
-__device__ __forceinline__ void filterHit(FitLane<FORM, MAT> &L, const Params &P,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void filterHit(FitLane<FORM, MAT, H> &L, const Params &P,
                                           const PlaneD *planes, int k) {
   const PlaneD &pl = planes[k];
   const int s = L.measStates;
   const bool first = s == 0;
-  const bool states = !MAT && P.oSmoothed != nullptr; // (with material: kf_device.cuh's lane)
-  const bool time = first || states;
+  using LT = FitLane<FORM, MAT, H>;
+  const bool states = !MAT && !LT::kTape && P.oSmoothed != nullptr; // (with material: kf_device.cuh's lane)
+  const bool time = (first || states) && !LT::kTape;
   double J[4][5], J5[5] = {0., 0., 0., 0., 0.};
   Trig tr;
   boundJacobian(L, P, planes, pl, time, tr, J, J5);
@@ -1166,6 +1175,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT> &L, const Params &P
         }
       }
     }
+    if constexpr (LT::kTape) L.hook.event(L, k, tr, J, x0, x1);
     if (time) {
       // x_p - F D, F
       double x[6] = {x0, x1, 0., 0., L.qop, L.t};
@@ -1395,6 +1405,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT> &L, const Params &P
   }
   // reinitializeJacobians (CovarianceEngine.hpp:169-201): at the predicted
   // direction, or with faithful_jacobian = 0 at the filtered one
+  if constexpr (LT::kTape) L.hook.eventEnd(outlier, tn);
   const Trig &tg = (P.faithful || outlier) ? tr : tn;
   trigSave(L, tg);
   legReset(L, tg);
@@ -1406,8 +1417,8 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT> &L, const Params &P
 // Actor::finalize (KalmanFitter.hpp:360-393): the smoothed first state
 // becomes the stepper's; false where the smoother's gain is NaN
 // ---------------------------------------------------------------------------
-template <int FORM, bool MAT>
-__device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT> &L, const Params &P,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT, H> &L, const Params &P,
                                                const PlaneD *planes) {
   L.smoothed = true;
   if (L.badJ) return false;
@@ -1474,10 +1485,10 @@ __device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT> &L, const Para
 }
 
 // boundState<LineSurface> towards the perigee line (axis z) and the outputs
-template <int FORM, bool MAT>
-__device__ __forceinline__ void reachPerigee(FitLane<FORM, MAT> &L, const Params &P,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void reachPerigee(FitLane<FORM, MAT, H> &L, const Params &P,
                                              const PlaneD *planes) {
-  using LT = FitLane<FORM, MAT>;
+  using LT = FitLane<FORM, MAT, H>;
   const Trig tl = trigLoad(L);
   double pg[3], dg[3], out[6], cov[21];
   toGlobal<LT>(P, L.pos, pg);
@@ -1682,10 +1693,10 @@ __device__ __forceinline__ void reachPerigee(FitLane<FORM, MAT> &L, const Params
 // EigenStepper::State from BoundParameters<LineSurface> (EigenStepper.hpp:40-61)
 // and the navigator initialisation
 // ---------------------------------------------------------------------------
-template <int FORM, bool MAT>
-__device__ __forceinline__ void initFit(FitLane<FORM, MAT> &L, const Params &P, const PlaneD *planes,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void initFit(FitLane<FORM, MAT, H> &L, const Params &P, const PlaneD *planes,
                                         int64_t i, int64_t wsIdx) {
-  using LT = FitLane<FORM, MAT>;
+  using LT = FitLane<FORM, MAT, H>;
   L.idx = i;
   L.wsIdx = wsIdx;
   L.pc = PC_DONE;
@@ -1779,8 +1790,8 @@ __device__ __forceinline__ void initFit(FitLane<FORM, MAT> &L, const Params &P, 
 // final transport can be due, and returns false without touching the state
 // otherwise.
 // ---------------------------------------------------------------------------
-template <int FORM, bool MAT>
-__device__ __forceinline__ bool actor(FitLane<FORM, MAT> &L, const Params &P, const PlaneD *planes,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ bool actor(FitLane<FORM, MAT, H> &L, const Params &P, const PlaneD *planes,
                                       bool heavy) {
   const bool onPlane = L.current >= 0 && !L.smoothed && !L.finished;
   const bool hit = onPlane && ((L.mask >> L.current) & 1ull);
@@ -1838,14 +1849,14 @@ __device__ __forceinline__ bool actor(FitLane<FORM, MAT> &L, const Params &P, co
 
 // Kalman aborter (KalmanFitter.hpp:682-694); the path limit
 // (StandardAborters.hpp:37-56) is DBL_MAX here and never reached
-template <int FORM, bool MAT>
-__device__ __forceinline__ bool aborters(FitLane<FORM, MAT> &L, const Params &) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ bool aborters(FitLane<FORM, MAT, H> &L, const Params &) {
   return !L.result || L.finished || L.targetReached;
 }
 
 // the pending actor call, and the rest of its iteration (see advance)
-template <int FORM, bool MAT>
-__device__ __forceinline__ void runEvent(FitLane<FORM, MAT> &L, const Params &P, const PlaneD *planes) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ void runEvent(FitLane<FORM, MAT, H> &L, const Params &P, const PlaneD *planes) {
   L.parked = false;
   actor(L, P, planes, true);
   if (L.pc == PC_POST) {
