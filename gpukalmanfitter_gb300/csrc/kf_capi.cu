@@ -114,7 +114,7 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
       F.invw[a] = (field->kind == KF_FIELD_GRID_RZ && a == 1)
                       ? 0.
                       : (na - 1) / (field->max[a] - field->min[a]);
-      F.off[a] = -F.mn[a] * F.invw[a] - 0.5;
+      F.off[a] = -F.mn[a] * F.invw[a];
     }
   }
   F.grid = reinterpret_cast<const float4 *>(field->grid);
@@ -141,6 +141,10 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
       pl.U[r] = geo->rotation[9 * k + 3 * r + 0];
       pl.V[r] = geo->rotation[9 * k + 3 * r + 1];
       pl.T[r] = geo->rotation[9 * k + 3 * r + 2];
+    }
+    for (int r = 0; r < 3; ++r) {
+      pl.Uf[r] = (float)pl.U[r];
+      pl.Vf[r] = (float)pl.V[r];
     }
     pl.tc = pl.T[0] * pl.c[0] + pl.T[1] * pl.c[1] + pl.T[2] * pl.c[2];
     {

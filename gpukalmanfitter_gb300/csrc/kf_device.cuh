@@ -54,7 +54,8 @@ constexpr int kStateStride = 37; // doubles per stored measurement state
 
 struct PlaneD {
   double c[3], U[3], V[3], T[3];
-  double tc; // T . c
+  double tc;          // T . c
+  float Uf[3], Vf[3]; // FP32 copies for the mixed form
 };
 
 struct FieldD {
@@ -62,7 +63,7 @@ struct FieldD {
   int n[3];
   double B[3]; // constant field, scale applied
   double scale;
-  double mn[3], invw[3], off[3]; // off = -mn invw - 1/2
+  double mn[3], invw[3], off[3]; // off = -mn invw
   const float4 *grid;
   float Bf[3], mnf[3], invwf[3], scalef; // FP32 copies for the mixed form
   float Blo[3], wf[3], scalelo;          // mixed form: lo parts of B and scale, cell width
@@ -114,6 +115,13 @@ __device__ __forceinline__ void cross3(const T a[3], const T b[3], T r[3]) {
 // std::max / std::min argument semantics (NaN handling as in the reference)
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
+
+// an FP32 value as FP64 on the integer pipe (normal values exactly; FP32
+// zeros and denormals come out below 1.2e-38)
+__device__ __forceinline__ double widen(float f) {
+  const int b = __float_as_int(f);
+  return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
+}
 
 enum { kAccuracy = 0, kActor = 1, kAborter = 2, kUser = 3 };
 enum { kMissed = 0, kReachable = 1, kOnSurface = 2 };
@@ -630,7 +638,7 @@ __device__ __forceinline__ void rkFirstDelta(const FieldD &F, const float posf[3
   double B[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    B[i] = kff::join(S.Bf[i]);
+    B[i] = widen(S.Bf[i].hi) + widen(S.Bf[i].lo);
     S.s.Bf[i] = S.Bf[i].hi;
   }
   double c[3];

@@ -112,6 +112,7 @@ template <> struct LegState<kMixed> {};
 struct NoBlocks {};
 struct MixedBlocks {
   float JA[3][3], Ja[3], Jb, JB[3][3], Jc[3], k4[3];
+  float qopf, d37f; // of the leg
   double sTr;
 };
 
@@ -204,11 +205,13 @@ template <class LT> __device__ __forceinline__ double *recPtr(const Params &P, c
 template <class LT>
 __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, bool time) {
   L.qop = L.q * ip;
+  if constexpr (LT::kForm == kMixed) L.qopf = (float)L.qop;
   if (time) {
     const double x = P.mass * ip, a = fma(x, x, 1.);
     const double y = rsqrtFast(a);
     L.dtds = a * y;
     L.d37 = P.mass * P.mass * L.qop * y;
+    if constexpr (LT::kForm == kMixed) L.d37f = (float)L.d37;
   }
 }
 
@@ -363,11 +366,15 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kUni
   stepUniform(L, P);
 }
 
-// an FP32 value as FP64 on the integer pipe (normal values exactly; FP32
-// zeros and denormals come out below 1.2e-38)
-__device__ __forceinline__ double widen(float f) {
-  const int b = __float_as_int(f);
-  return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
+// 1/|d| for |d|^2 = 1 + e: one Newton step of 1/sqrt from 1 (error 3/8 e^2)
+// where e is below 1e-8, as in all but steps that turn far
+__device__ __forceinline__ double unitFactor(const double d[3]) {
+  const double n2 = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
+  const double f = fma(n2, -0.5, 1.5);
+  // 1 +- 1e-8 by the bits of 3/2 - n2/2
+  const long long k = __double_as_longlong(f) - 0x3ff0000000000000LL;
+  if (k > 22517998LL || k < -45035996LL) return rsqrt(n2);
+  return f;
 }
 
 // field at p times s (s = scale q/p), FP64 trilinear: the lookup of getField
@@ -392,11 +399,10 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
   double f[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    // the cell's middle rounds to its index: floor by adding 2^52 + 2^51 to
-    // the coordinate less 1/2; a tie (a point on a grid plane) may give the
-    // cell below, whose upper corner it then is
+    // floor by adding 2^52 + 2^51, whose unit in the last place is 1, with
+    // rounding down
     const double gr = fma(p[a], F.invw[a], F.off[a]);
-    const double t = gr + 6755399441055744.;
+    const double t = __dadd_rd(gr, 6755399441055744.);
     int i = __double2loint(t);
     double fi = t - 6755399441055744.;
     const int lim = F.n[a] - 2;
@@ -405,7 +411,7 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
       fi = (double)i;
     }
     idx[a] = i;
-    f[a] = (gr - fi) + 0.5;
+    f[a] = gr - fi;
   }
   const size_t nx = F.n[0], nxy = (size_t)F.n[0] * F.n[1];
   const float4 *g = F.grid + ((size_t)idx[2] * nxy + (size_t)idx[1] * nx + idx[0]);
@@ -509,11 +515,7 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
     L.dir[i] = fma(h6, fma(2., s23, k1[i] + k4[i]), L.dir[i]);
     g.k4[i] = k4[i];
   }
-  // |dir|^2 = 1 + e, e ~ (h kappa)^4: two Newton steps of 1/sqrt from 1
-  const double n2 = L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1] + L.dir[2] * L.dir[2];
-  double f = 1.5 - 0.5 * n2;
-  f = f * (1.5 - 0.5 * n2 * f * f);
-  if (fabs(n2 - 1.) > 1e-4) f = 1. / sqrt(n2); // large turning steps
+  const double f = unitFactor(L.dir);
   L.dir[0] *= f;
   L.dir[1] *= f;
   L.dir[2] *= f;
@@ -533,16 +535,18 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
 template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMixed, MAT, H> &L, const Params &P) {
   long nTrials = 0;
   double h = ssValue(L);
-  const float qopf = (float)L.qop;
+  const float qopf = L.qopf;
   const float posf[3] = {(float)L.pos[0], (float)L.pos[1], (float)L.pos[2]};
-  const float res[3] = {(float)(L.pos[0] - (double)posf[0]), (float)(L.pos[1] - (double)posf[1]),
-                        (float)(L.pos[2] - (double)posf[2])};
+  const float res[3] = {(float)(L.pos[0] - widen(posf[0])), (float)(L.pos[1] - widen(posf[1])),
+                        (float)(L.pos[2] - widen(posf[2]))};
+  float hf;
   const float dirf[3] = {(float)L.dir[0], (float)L.dir[1], (float)L.dir[2]};
   StagesDelta S;
   rkFirstDelta(P.field, posf, res, L.dir, L.qop, S);
   for (;;) {
     L.rkTrials++;
-    const float errf = rkTrialDelta(P.field, posf, res, dirf, qopf, (float)h, S);
+    hf = (float)h;
+    const float errf = rkTrialDelta(P.field, posf, res, dirf, qopf, hf, S);
     if (errf <= P.tolLoF) break;
     RkStages<double> sd;
     rkFirst<double>(P.field, L.pos, L.dir, L.qop, sd);
@@ -550,7 +554,7 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMix
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) return;
   }
-  transportUpdate<float>(L, dirf, qopf, (float)h, (float)L.d37, S.s);
+  transportUpdate<float>(L, dirf, qopf, hf, L.d37f, S.s);
   L.sTr += h;
   // motion: FP64 state, FP64 k1, FP32 sums of the offsets
   //   pos += h d + h^2/6 (3 k1 + d2 + d3),  dir += h/6 (6 k1 + 2 (d2 + d3) + d4)
@@ -559,15 +563,10 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMix
   for (int i = 0; i < 3; ++i) {
     const float s23 = S.d2[i] + S.d3[i];
     const float s234 = 2.f * s23 + S.d4[i];
-    L.pos[i] = L.pos[i] + (h * L.dir[i] + hh6 * (3. * S.k1[i] + widen(s23)));
-    L.dir[i] = L.dir[i] + h6 * (6. * S.k1[i] + widen(s234));
+    L.pos[i] = fma(hh6, fma(3., S.k1[i], widen(s23)), fma(h, L.dir[i], L.pos[i]));
+    L.dir[i] = fma(h6, fma(6., S.k1[i], widen(s234)), L.dir[i]);
   }
-  // |dir|^2 = 1 + e with e ~ (h kappa)^2 <= 1e-3: two Newton steps of
-  // 1/sqrt from 1 reach FP64 precision (error ~ e^4)
-  const double n2 = L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1] + L.dir[2] * L.dir[2];
-  double f = 1.5 - 0.5 * n2;
-  f = f * (1.5 - 0.5 * n2 * f * f);
-  if (fabs(n2 - 1.) > 1e-3) f = 1. / sqrt(n2); // large turning steps
+  const double f = unitFactor(L.dir);
   L.dir[0] *= f;
   L.dir[1] *= f;
   L.dir[2] *= f;
@@ -866,14 +865,17 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
     for (int r = 0; r < 3; ++r) {
       P0[r][0] = U[r];
       P0[r][1] = V[r];
-      P0[r][2] = (r < 2 ? o2[r] : 0.) + s * g46[r][0];
+      P0[r][2] = r < 2 ? fma(s, g46[r][0], o2[r]) : 0.;
       P0[r][3] = s * g46[r][1];
     }
   }
   // ---- straight-line part, FP64
   const double nv[3] = {pl.T[0] * L.idn, pl.T[1] * L.idn, pl.T[2] * L.idn};
 #pragma unroll
-  for (int c = 0; c < 4; ++c) s0[c] = nv[0] * P0[0][c] + nv[1] * P0[1][c] + nv[2] * P0[2][c];
+  for (int c = 0; c < 4; ++c) { // (the phi column, c = 2, has no z)
+    const double col[3] = {P0[0][c], P0[1][c], P0[2][c]};
+    s0[c] = dotz(c == 2, nv, col);
+  }
   double A0[3], A1[3];
   {
     const double u0 = st ? dot3(pl.U, L.dir) : 0., u1 = st ? dot3(pl.V, L.dir) : 0.;
@@ -887,12 +889,13 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
   const double j34 = tr.cP * tr.cT, j35 = tr.sP * tr.cT, j36 = -tr.sT;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    J[0][c] = A0[0] * P0[0][c] + A0[1] * P0[1][c] + A0[2] * P0[2][c];
-    J[1][c] = A1[0] * P0[0][c] + A1[1] * P0[1][c] + A1[2] * P0[2][c];
+    const double col[3] = {P0[0][c], P0[1][c], P0[2][c]};
+    J[0][c] = dotz(c == 2, A0, col);
+    J[1][c] = dotz(c == 2, A1, col);
     if (c >= 2) {
       const double g0 = g46[0][c - 2], g1 = g46[1][c - 2], g2 = g46[2][c - 2];
-      J[2][c] = j24 * g0 + j25 * g1;
-      J[3][c] = j34 * g0 + j35 * g1 + j36 * g2;
+      J[2][c] = fma(j24, g0, j25 * g1);
+      J[3][c] = fma(j34, g0, c == 2 ? j35 * g1 : fma(j35, g1, j36 * g2));
     } else {
       J[2][c] = 0.;
       J[3][c] = 0.;
@@ -942,8 +945,7 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
 #pragma unroll
     for (int c = 0; c < 5; ++c) R3[c] = (c == 4 ? L.Jb : 0.f);
   }
-  const float U[3] = {(float)pl.U[0], (float)pl.U[1], (float)pl.U[2]};
-  const float V[3] = {(float)pl.V[0], (float)pl.V[1], (float)pl.V[2]};
+  const float *U = pl.Uf, *V = pl.Vf;
   const float f24 = (float)j24, f25 = (float)j25, f34 = (float)j34, f35 = (float)j35, f36 = (float)j36;
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
