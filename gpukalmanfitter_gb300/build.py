@@ -23,7 +23,7 @@ LIB = LIBDIR / "libgb300kf.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # fit kernels: one file per precision and register budget
 CU_SOURCES = ["kf_capi.cu", "kf_launch.cu", "kf_batch.cu", "kf_fit_material.cu",
-              "kf_fit_material_states.cu", "kf_fit_fp64_any.cu", "kf_diag.cu", "kf_noalloc.cu", "kf_adjoint.cu",
+              "kf_fit_material_states.cu", "kf_fit_fp64_any.cu", "kf_fit_coop.cu", "kf_diag.cu", "kf_noalloc.cu", "kf_adjoint.cu",
               "kf_adjoint_z.cu",
               "kf_sim.cu"] + [f"kf_fit_{p}_{r}.cu" for p in ("fp64", "mixed")
                               for r in (255, 168, 128, 96)]

@@ -53,7 +53,8 @@ enum {
 static_assert(zWords <= 2 * kStateStride, "state record");
 
 struct ZHook {
-  static constexpr bool kMaterial = false;
+  static constexpr bool kTape = true;
+  static constexpr int kGroup = 1;
   double *tape;       // this lane's word 0; word k at tape[k * n]
   double *recA, *recB;
   int32_t *info;

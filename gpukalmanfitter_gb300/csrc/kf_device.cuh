@@ -321,6 +321,8 @@ template <typename R> __host__ __device__ constexpr size_t coldStateBytes(int th
 // to nothing); the chi2 adjoint records its tape through these calls.
 struct NoHook {
   static constexpr bool kMaterial = false; // surface material code compiled in
+  static constexpr bool kTape = false;     // kf_fit.cuh: the adjoint's forward pass
+  static constexpr int kGroup = 1;         // kf_fit.cuh: lanes of a warp per track
   template <class LT> __device__ __forceinline__ void stepBegin(const LT &) {}
   template <class LT> __device__ __forceinline__ void trial(const LT &, double) {}
   template <class LT> __device__ __forceinline__ void stepEnd(const LT &, bool) {}

@@ -94,7 +94,11 @@ __host__ __device__ constexpr int u5(int i, int j) { // upper triangle of 5x5
 enum { kRecX = 0, kRecF = 6, kRecT = 26, kRecTrig = 31 };
 static_assert(kRecTrig + 4 <= kStateStride, "state record");
 
-template <int FORM> struct LegState;
+template <int FORM, int GROUP = 1> struct LegState;
+// eight lanes on one track (kf_fit_coop.cuh)
+struct CoopHook : NoHook {
+  static constexpr int kGroup = 8;
+};
 // uniform field, z along the field: with A v = v x z the leg's transport is
 // dir: I + b A + (1 - g) A^2, pos: s I + q1 A + (s - r) A^2; c, a: q/p column
 template <> struct LegState<kUniform64> {
@@ -109,6 +113,12 @@ template <> struct LegState<kGrid64> {
 // mixed: FP32 transport blocks as offsets from the straight line
 // (applyTransportOffsets)
 template <> struct LegState<kMixed> {};
+template <> struct LegState<kUniform64, 8> : LegState<kUniform64> {};
+template <> struct LegState<kMixed, 8> {};
+// each lane of a group carries its own column (2: phi, 3: theta, 4: q/p)
+template <> struct LegState<kGrid64, 8> {
+  double p[3], v[3], s, k4[3];
+};
 struct NoBlocks {};
 struct MixedBlocks {
   float JA[3][3], Ja[3], Jb, JB[3][3], Jc[3], k4[3];
@@ -120,13 +130,14 @@ template <int FORM, bool MAT_, class H_ = NoHook>
 struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
   static constexpr int kForm = FORM;
   static constexpr bool kMat = MAT_;
-  static constexpr bool kTape = !std::is_same<H_, NoHook>::value; // the adjoint's forward pass
+  static constexpr bool kTape = H_::kTape;
+  static constexpr bool kCoop = H_::kGroup > 1;
   double pos[3], dir[3]; // FP64 uniform field: in the field's frame
   double q, qop, t, dtds, d37;
   double idn;            // 1 / (T . dir) of the plane last looked at
   double ss[4];
   int ssDir, navDir;
-  LegState<FORM> g;
+  LegState<FORM, H_::kGroup> g;
   bool stepped;
   int next, current, nSeq, navCache, navCacheSt;
   long long navCacheLim;
@@ -141,16 +152,29 @@ struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
   __device__ __forceinline__ double &cold(int e) const {
     return reinterpret_cast<double *>(kfColdSmem)[e * blockDim.x + threadIdx.x];
   }
-  // no process noise
-  __device__ __forceinline__ double &F(int r, int c) const { return cold(5 * r + c); }
-  __device__ __forceinline__ double &C0(int e) const { return cold(20 + e); }
+  // the column of lane l of this thread's group
+  __device__ __forceinline__ double &coldOf(int e, int l) const {
+    return reinterpret_cast<double *>(kfColdSmem)[e * blockDim.x + (threadIdx.x & ~(H_::kGroup - 1)) + l];
+  }
+  // no process noise; in a group, lane c holds column c of F, row c of C0's
+  // upper triangle and entry c of D
+  __device__ __forceinline__ double &F(int r, int c) const {
+    return kCoop ? coldOf(r, c) : cold(5 * r + c);
+  }
+  __device__ __forceinline__ double &C0(int e) const {
+    if (!kCoop) return cold(20 + e);
+    const int i = e < 5 ? 0 : e < 9 ? 1 : e < 12 ? 2 : e < 14 ? 3 : 4;
+    return coldOf(4 + e - u5(i, i), i);
+  }
   __device__ __forceinline__ double &Ct(int i) const { return cold(35 + i); }
   // process noise
   __device__ __forceinline__ double &C(int e) const { return cold(e); }
   __device__ __forceinline__ double &X(int r, int c) const { return cold(15 + 5 * r + c); }
   __device__ __forceinline__ double &P1(int e) const { return cold(45 + e); }
   // both: D (sum of K0 r) and the trigonometry (cos phi, sin phi, cos theta, sin theta)
-  __device__ __forceinline__ double &D(int i) const { return cold((MAT_ ? 66 : 41) + i); }
+  __device__ __forceinline__ double &D(int i) const {
+    return kCoop && i < 5 ? coldOf(9, i) : cold((MAT_ ? 66 : 41) + i);
+  }
   __device__ __forceinline__ double &trigS(int i) const { return cold((MAT_ ? 72 : 47) + i); }
 };
 
@@ -226,6 +250,15 @@ __device__ __forceinline__ void legReset(FitLane<FORM, MAT, H> &L, const Trig &t
     L.g.b = L.g.r = L.g.q1 = L.g.s = 0.;
     L.g.c[0] = L.g.c[1] = L.g.a[0] = L.g.a[1] = 0.;
     L.g.y = L.g.dx = L.g.dy = 0.;
+  } else if constexpr (FORM == kGrid64 && H::kGroup > 1) {
+    const int c = threadIdx.x & 7;
+    const bool phi = c == 2, th = c == 3;
+    L.g.p[0] = L.g.p[1] = L.g.p[2] = 0.;
+    L.g.v[0] = phi ? -t.sT * t.sP : (th ? t.cT * t.cP : 0.);
+    L.g.v[1] = phi ? t.sT * t.cP : (th ? t.cT * t.sP : 0.);
+    L.g.v[2] = th ? -t.sT : 0.;
+    L.g.s = 0.;
+    L.g.k4[0] = L.g.k4[1] = L.g.k4[2] = 0.;
   } else if constexpr (FORM == kGrid64) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -477,35 +510,41 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
   const double hh = 0.5 * h, h6 = h * (1. / 6.), hh6 = h * h6;
   const double iq = rcpFast(L.qop);
   auto &g = L.g;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
+  auto column = [&](double (&p)[3], double (&v)[3], bool own, double q1) {
     double e1[3], e2[3], e3[3], e4[3], w[3];
     auto src = [&](double e[3], const double k[3]) {
-      if (c == 2) {
+      if (own) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) e[i] = fma(k[i], iq, e[i]);
+        for (int i = 0; i < 3; ++i) e[i] = fma(k[i], q1, e[i]);
       }
     };
-    cross3(g.v[c], b1, e1);
+    cross3(v, b1, e1);
     src(e1, k1);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) w[i] = fma(hh, e1[i], g.v[c][i]);
+    for (int i = 0; i < 3; ++i) w[i] = fma(hh, e1[i], v[i]);
     cross3(w, b2, e2);
     src(e2, k2);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) w[i] = fma(hh, e2[i], g.v[c][i]);
+    for (int i = 0; i < 3; ++i) w[i] = fma(hh, e2[i], v[i]);
     cross3(w, b2, e3);
     src(e3, k3);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) w[i] = fma(h, e3[i], g.v[c][i]);
+    for (int i = 0; i < 3; ++i) w[i] = fma(h, e3[i], v[i]);
     cross3(w, b3, e4);
     src(e4, k4);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const double s23 = e2[i] + e3[i];
-      g.p[c][i] = fma(hh6, e1[i] + s23, fma(h, g.v[c][i], g.p[c][i]));
-      g.v[c][i] = fma(h6, fma(2., s23, e1[i] + e4[i]), g.v[c][i]);
+      p[i] = fma(hh6, e1[i] + s23, fma(h, v[i], p[i]));
+      v[i] = fma(h6, fma(2., s23, e1[i] + e4[i]), v[i]);
     }
+  };
+  if constexpr (H::kGroup > 1) {
+    column(g.p, g.v, true, (threadIdx.x & 7) == 4 ? iq : 0.);
+  } else {
+    column(g.p[0], g.v[0], false, 0.);
+    column(g.p[1], g.v[1], false, 0.);
+    column(g.p[2], g.v[2], true, iq);
   }
   g.s += h;
 #pragma unroll
@@ -700,8 +739,14 @@ __device__ __forceinline__ void legColumn(const FitLane<kGrid64, MAT, H> &L, con
                                           const Trig &t, double o, int c, double p[3], double v[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    p[i] = L.g.p[c - 2][i];
-    v[i] = L.g.v[c - 2][i];
+    if constexpr (H::kGroup > 1) { // from the lane that carries it (the whole group calls)
+      const unsigned group = 0xffu << (threadIdx.x & 24);
+      p[i] = __shfl_sync(group, L.g.p[i], c, 8);
+      v[i] = __shfl_sync(group, L.g.v[i], c, 8);
+    } else {
+      p[i] = L.g.p[c - 2][i];
+      v[i] = L.g.v[c - 2][i];
+    }
   }
   if (c == 2 && L.measStates == 0) {
     p[0] -= o * t.cP;

@@ -17,15 +17,15 @@
 // so that every shape of one budget, queue or not, gives the same bits.
 #pragma once
 
-#include "kf_fit.cuh"
+#include "kf_fit_coop.cuh"
 
 namespace kfd {
 
 // Fit the tracks i (inputs/outputs) with workspace columns w of one warp;
 // i < 0 marks an idle lane.  All 32 lanes must call it together.
-template <int FORM, bool MAT>
+template <int FORM, bool MAT, class H = NoHook>
 __device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64_t i, int64_t w) {
-  FitLane<FORM, MAT> L;
+  FitLane<FORM, MAT, H> L;
   initFit(L, P, sp, i, w);
   for (;;) {
     if (!L.parked && L.pc != PC_DONE) advance(L, P, sp);
@@ -35,7 +35,7 @@ __device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64
       if (__all_sync(0xffffffffu, L.pc == PC_DONE)) break;
     }
   }
-  if (i >= 0 && i < P.n) {
+  if (i >= 0 && i < P.n && (threadIdx.x & (H::kGroup - 1)) == 0) {
     P.oStatus[i] = L.status;
     P.oChi2[i] = L.chi2;
     P.oNMeas[i] = L.measStates;
@@ -75,7 +75,24 @@ __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ 
   }
 }
 
+// P.lanes (1 ... 4) tracks a warp, eight lanes each (kf_fit_coop.cuh).
+template <int FORM> __global__ void __launch_bounds__(32, 8) fitCoop(const __grid_constant__ Params P) {
+  PlaneD *sp = reinterpret_cast<PlaneD *>(kfColdSmem + (size_t)blockDim.x * coldSlots<false>() * sizeof(double));
+  for (int k = threadIdx.x; k < P.nSurf; k += blockDim.x) sp[k] = P.planes[k];
+  __syncthreads();
+  const int g = threadIdx.x >> 3;
+  const int64_t i = (int64_t)blockIdx.x * P.lanes + g;
+  const bool own = g < P.lanes && i < P.n;
+  fitWarp<FORM, false, CoopHook>(P, sp, own ? i : -1, own ? i : 0);
+}
+
 } // namespace kfd
+
+#define KF_COOP_LAUNCHER(NAME, FORM)                                                           \
+  cudaError_t NAME(const kfd::Params &P, int, cudaStream_t s) {                              \
+    kfd::fitCoop<FORM><<<(unsigned)((P.n + P.lanes - 1) / P.lanes), 32, kfd::fitSmemBytes<false>(32, P.nSurf), s>>>(P); \
+    return cudaGetLastError();                                                               \
+  }
 
 // Launcher of one instantiation: bs threads per block; with a queue as many
 // blocks as the device holds at once, never more than the batch needs.

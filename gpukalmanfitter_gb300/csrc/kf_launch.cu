@@ -19,6 +19,9 @@ KF_DECLARE(launchFitMaterial_fp64_any)
 KF_DECLARE(launchFitMaterial_fp64_uniform)
 KF_DECLARE(launchFitMaterial_fp64_grid)
 KF_DECLARE(launchFitMaterial_mixed)
+KF_DECLARE(launchFitCoop_fp64_uniform)
+KF_DECLARE(launchFitCoop_fp64_grid)
+KF_DECLARE(launchFitCoop_mixed)
 KF_DECLARE(launchFitMaterialStates_fp64)
 KF_DECLARE(launchFitMaterialStates_mixed)
 
@@ -108,6 +111,8 @@ static void toFieldFrame(Params &P) {
   }
 }
 
+constexpr int64_t kLeastWarps = 3; // warps an SM that a small batch spreads over
+
 // How a batch is laid over the chip.  One FP64 instruction of a warp costs the
 // same whatever its active lanes, each SM sub-partition starts one every 64
 // cycles, and four warps (one a sub-partition) fill an SM's FP64 pipe.  So a
@@ -124,11 +129,17 @@ struct Spread {
 static Spread spread(int64_t n, int sms) {
   if (n > 0x7f000000) return {32, false, false}; // the queue counts in 32 bits
   const int64_t full = 32 * (int64_t)sms;
-  const int64_t perSm = std::max<int64_t>(3, (n + full - 1) / full);
+  const int64_t perSm = std::max<int64_t>(kLeastWarps, (n + full - 1) / full);
   if (perSm > 8) return {32, true, true};
   const int lanes = (int)((n + sms * perSm - 1) / (sms * perSm));
   return {lanes, lanes >= 8, false};
 }
+
+// Batches of up to kCoopMost tracks an SM run eight lanes a track, again as few
+// tracks a warp as kLeastWarps warps an SM allow (the line is where five such
+// warps of four tracks an SM cost as much as 3 warps of 7 lanes: 3000 tracks of
+// 10 planes 418 against 458 us, 3600 tracks 503 against 485 us).
+constexpr int64_t kCoopMost = 20;
 
 int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers &q, cudaStream_t s) {
   const bool mixed = precision == KF_PRECISION_MIXED;
@@ -145,6 +156,14 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cudaFail(e, "device query");
   const bool asked = (bs || minb) && !P.materialEffects; // a requested shape: always the queue
+  const bool uniform = P.field.kind == KF_FIELD_CONSTANT;
+  const bool offAxis = !mixed && uniform && (P.field.B[0] != 0. || P.field.B[1] != 0.);
+  if (!asked && !P.materialEffects && !P.oSmoothed && !offAxis && P.n <= kCoopMost * sms) {
+    if (!mixed && uniform) toFieldFrame(P);
+    P.lanes = (int)std::min<int64_t>(4, (P.n + kLeastWarps * sms - 1) / (kLeastWarps * sms));
+    e = (mixed ? launchFitCoop_mixed : uniform ? launchFitCoop_fp64_uniform : launchFitCoop_fp64_grid)(P, 0, s);
+    return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
+  }
   Spread sp = spread(P.n, sms);
   if (asked) sp = {32, P.n > kSortBuckets, P.n > kSortBuckets};
   P.lanes = sp.lanes;
@@ -158,7 +177,7 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   const int block = asked ? shape->bs : kDefaultBlock;
   if (mixed) {
     e = b->mixed(P, block, s);
-  } else if (P.field.kind != KF_FIELD_CONSTANT) {
+  } else if (!uniform) {
     e = b->grid(P, block, s);
   } else {
     toFieldFrame(P);

@@ -107,3 +107,20 @@ def test_material_forms(kf, orc, kw):
     rep = parity_report(g, o, TOL, mask=o["status"] == 0)
     print(rep)
     assert rep["params"] <= 1 and rep["chi2"] <= 1 and rep["cov"] <= 10, rep
+
+
+@pytest.mark.parametrize("n", [1, 3, 5, 31, 700, 3041])
+@pytest.mark.parametrize("kind", ["uniform", "map", "mixed"])
+def test_lanes_per_track_do_not_change_the_bits(kf, n, kind):
+    """Small batches run eight lanes a track, larger ones a lane a track with
+    fewer or more tracks a warp, in or out of order: the first n tracks of a
+    larger batch come out bitwise as a batch of n does."""
+    kw = dict(n_planes=15, x_first=80., x_step=80., min_len=5, max_len=15, hit_prob=0.9,
+              outlier_prob=0.02, field_map=kind == "map")
+    tel = _correlate_time(kf.make_telescope(6000, seed=35, **kw))
+    from gpukalmanfitter_gb300 import shard
+    cfg = kf.default_config(overstep_limit=0.1, outlier_chi2_cut=25.0, precision=int(kind == "mixed"))
+    whole = kf.fit_device(tel, cfg)
+    part = kf.fit_device(shard.subset(tel, np.arange(n)), cfg)
+    for k, v in part.items():
+        assert np.array_equal(v, whole[k][..., :n]), k
