@@ -130,6 +130,8 @@ void fillParams(Params &P, const kf_inputs_t *in, const kf_outputs_t *out, const
   P.tolLoF = (float)(P.tol * 0.99);
   // below the reference's floor of the error estimate (1e-20) FP64 decides
   P.tolAcceptF = P.tol > 1e-19 ? (float)(P.tol * (1. - 1e-5)) : -1.f;
+  P.cutKey = -1;
+  if (P.outlierCut > 0.) std::memcpy(&P.cutKey, &P.outlierCut, sizeof(double));
   // |A d + y A^2 d|_1 <= sqrt(3) (1 + |y|) |d|, |y| <= 0.1: err <= 0.4764 |h y x|
   const double bound = P.tol > 1e-19 ? P.tol / 0.477 : -1.;
   P.errBound = bound < 0. ? -1 : 0;

@@ -76,6 +76,7 @@ struct Params {
   double tol, cutoff, mass, overstep, surfTol, outlierCut;
   float tolLoF;         // mixed form: FP32 error estimates up to this accept
   float tolAcceptF;     // FP64 map form: FP32-rounded error estimates up to this accept
+  long long cutKey;     // outlierCut's bits, -1 for none
   long long errBound;   // FP64 uniform form: |h y x| up to this (bits of a double) accept
   const double *meas;
   const uint64_t *mask;
@@ -121,6 +122,30 @@ __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b 
 __device__ __forceinline__ double widen(float f) {
   const int b = __float_as_int(f);
   return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
+}
+
+// FP64 to FP32, rounded to nearest even, on the integer pipe (a conversion
+// takes the FP64 pipe as long as an FMA); results below the least normal FP32
+// value come out as zero
+__device__ __forceinline__ float narrow(double d) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+  const unsigned long long r = b + (0x0fffffffu + ((unsigned)(b >> 29) & 1u));
+  const unsigned a = (unsigned)(r >> 32) & 0x7fffffffu;
+  if (a >= 0x47f00000u) return (float)d; // beyond FP32, infinite or NaN
+  const unsigned f = a < 0x38100000u ? 0u : ((unsigned)(r >> 29) + 0x40000000u) & 0x7fffffffu;
+  return __uint_as_float(f | ((unsigned)(b >> 32) & 0x80000000u));
+}
+// d as narrow(d) and the FP32 rounding of the rest d - narrow(d), which is a
+// 29-bit integer in units of d's last place (0 for |d| below 2^-75)
+__device__ __forceinline__ void split(double d, float &f, float &rest) {
+  f = narrow(d);
+  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+  const unsigned lo = (unsigned)b & 0x1fffffffu;
+  const bool up = lo > 0x10000000u || (lo == 0x10000000u && ((b >> 29) & 1u));
+  const int n = (int)lo - (up ? 0x20000000 : 0);
+  const int e = (int)((b >> 52) & 0x7ffu) - (1075 - 127);
+  const unsigned s = (e > 0 ? (unsigned)e << 23 : 0u) | ((unsigned)(b >> 32) & 0x80000000u);
+  rest = __int2float_rn(n) * __uint_as_float(s);
 }
 
 enum { kAccuracy = 0, kActor = 1, kAborter = 2, kUser = 3 };
@@ -648,7 +673,7 @@ __device__ __forceinline__ void rkFirstDelta(const FieldD &F, const float posf[3
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     S.k1[i] = qop * c[i];
-    S.s.k1[i] = (float)S.k1[i];
+    S.s.k1[i] = narrow(S.k1[i]);
   }
 }
 

@@ -229,7 +229,7 @@ template <class LT> __device__ __forceinline__ double *recPtr(const Params &P, c
 template <class LT>
 __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, bool time) {
   L.qop = L.q * ip;
-  if constexpr (LT::kForm == kMixed) L.qopf = (float)L.qop;
+  if constexpr (LT::kForm == kMixed) L.qopf = narrow(L.qop);
   if (time) {
     const double x = P.mass * ip, a = fma(x, x, 1.);
     const double y = rsqrtFast(a);
@@ -302,6 +302,17 @@ __device__ __forceinline__ bool rejectTrial(LT &L, const Params &P, double err, 
   if (h * h < P.cutoff * P.cutoff || nTrials > P.maxTrials) return false;
   nTrials++;
   return true;
+}
+
+// 1/|d| for |d|^2 = 1 + e: one Newton step of 1/sqrt from 1 (error 3/8 e^2)
+// where e is below 1e-8, as in all but steps that turn far
+__device__ __forceinline__ double unitFactor(const double d[3]) {
+  const double n2 = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
+  const double f = fma(n2, -0.5, 1.5);
+  // 1 +- 1e-8 by the bits of 3/2 - n2/2
+  const long long k = __double_as_longlong(f) - 0x3ff0000000000000LL;
+  if (k > 22517998LL || k < -45035996LL) return rsqrt(n2);
+  return f;
 }
 
 // Uniform field along z.  With A v = v x z (A^3 = -A), y = h q/p B and
@@ -382,9 +393,7 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT, H> &L, const Para
   L.dir[0] = fma(be1, dx, al * dy);
   L.dir[1] = fma(be1, dy, -al * dx);
   if (!(akey(x) < 0x3ee4f8b588e368f1LL)) { // |x| >= 1e-5
-    const double n2 = L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1] + L.dir[2] * L.dir[2];
-    double f = fma(n2, -0.5, 1.5);
-    if (fabs(n2 - 1.) > 1e-9) f = rsqrt(n2); // large turning steps
+    const double f = unitFactor(L.dir);
     L.dir[0] *= f;
     L.dir[1] *= f;
     L.dir[2] *= f;
@@ -397,17 +406,6 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kUni
 }
 template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kUniformAny, MAT, H> &L, const Params &P) {
   stepUniform(L, P);
-}
-
-// 1/|d| for |d|^2 = 1 + e: one Newton step of 1/sqrt from 1 (error 3/8 e^2)
-// where e is below 1e-8, as in all but steps that turn far
-__device__ __forceinline__ double unitFactor(const double d[3]) {
-  const double n2 = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
-  const double f = fma(n2, -0.5, 1.5);
-  // 1 +- 1e-8 by the bits of 3/2 - n2/2
-  const long long k = __double_as_longlong(f) - 0x3ff0000000000000LL;
-  if (k > 22517998LL || k < -45035996LL) return rsqrt(n2);
-  return f;
 }
 
 // field at p times s (s = scale q/p), FP64 trilinear: the lookup of getField
@@ -575,16 +573,15 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMix
   long nTrials = 0;
   double h = ssValue(L);
   const float qopf = L.qopf;
-  const float posf[3] = {(float)L.pos[0], (float)L.pos[1], (float)L.pos[2]};
-  const float res[3] = {(float)(L.pos[0] - widen(posf[0])), (float)(L.pos[1] - widen(posf[1])),
-                        (float)(L.pos[2] - widen(posf[2]))};
-  float hf;
-  const float dirf[3] = {(float)L.dir[0], (float)L.dir[1], (float)L.dir[2]};
+  float posf[3], res[3], hf;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) split(L.pos[i], posf[i], res[i]);
+  const float dirf[3] = {narrow(L.dir[0]), narrow(L.dir[1]), narrow(L.dir[2])};
   StagesDelta S;
   rkFirstDelta(P.field, posf, res, L.dir, L.qop, S);
   for (;;) {
     L.rkTrials++;
-    hf = (float)h;
+    hf = narrow(h);
     const float errf = rkTrialDelta(P.field, posf, res, dirf, qopf, hf, S);
     if (errf <= P.tolLoF) break;
     RkStages<double> sd;
@@ -623,7 +620,7 @@ template <int FORM, bool MAT, class H>
 __device__ __forceinline__ int updateSurfaceStatus(FitLane<FORM, MAT, H> &L, const Params &P,
                                                    const PlaneD &pl, int k) {
   const double denom = pl.T[0] * L.dir[0] + pl.T[1] * L.dir[1] + pl.T[2] * L.dir[2];
-  if (denom != 0.0) {
+  if (akey(denom) != 0) {
     // along dir; the reference's path is along navDir * dir
     L.idn = rcpFast(denom);
     const double along =
@@ -656,7 +653,7 @@ __device__ __forceinline__ void lineIntersect(const FitLane<FORM, MAT, H> &L, co
                m2 = P.perigee[2 * P.stride + L.idx] - pg[2];
   const double denom = 1 - ea2 * ea2;
   if (denom * denom > P.surfTol * P.surfTol) {
-    u = ((m0 * ea0 + m1 * ea1 + m2 * ea2) - m2 * ea2) / denom;
+    u = ((m0 * ea0 + m1 * ea1 + m2 * ea2) - m2 * ea2) * rcpFast(denom);
     status = (u * u < P.surfTol * P.surfTol) ? kOnSurface : kReachable;
   } else {
     u = DBL_MAX;
@@ -950,8 +947,8 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
   float G[3][2];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    G[r][0] = (float)g46[r][0];
-    G[r][1] = (float)g46[r][1];
+    G[r][0] = narrow(g46[r][0]);
+    G[r][1] = narrow(g46[r][1]);
   }
   float dP[3][5], dD[3][5];
 #pragma unroll
@@ -965,16 +962,16 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
     dP[r][4] = L.Ja[r];
     dD[r][4] = L.Jc[r];
   }
-  const float nvf[3] = {(float)nv[0], (float)nv[1], (float)nv[2]};
+  const float nvf[3] = {narrow(nv[0]), narrow(nv[1]), narrow(nv[2])};
   float ds[5], sf[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
     ds[c] = nvf[0] * dP[0][c] + nvf[1] * dP[1][c] + nvf[2] * dP[2][c];
-    sf[c] = (c < 4 ? (float)s0[c] : 0.f) + ds[c];
+    sf[c] = (c < 4 ? narrow(s0[c]) : 0.f) + ds[c];
   }
   float R3[5];
   if (st) {
-    const float d0 = (float)L.dir[0], d1 = (float)L.dir[1], d2 = (float)L.dir[2];
+    const float d0 = narrow(L.dir[0]), d1 = narrow(L.dir[1]), d2 = narrow(L.dir[2]);
     const float dt = (float)L.dtds;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
@@ -991,7 +988,7 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
     for (int c = 0; c < 5; ++c) R3[c] = (c == 4 ? L.Jb : 0.f);
   }
   const float *U = pl.Uf, *V = pl.Vf;
-  const float f24 = (float)j24, f25 = (float)j25, f34 = (float)j34, f35 = (float)j35, f36 = (float)j36;
+  const float f24 = narrow(j24), f25 = narrow(j25), f34 = narrow(j34), f35 = narrow(j35), f36 = narrow(j36);
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
     const float e0 = U[0] * dP[0][c] + U[1] * dP[1][c] + U[2] * dP[2][c];
@@ -999,8 +996,10 @@ __device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, 
     const float e2 = f24 * dD[0][c] + f25 * dD[1][c];
     const float e3 = f34 * dD[0][c] + f35 * dD[1][c] + f36 * dD[2][c];
     const double w0 = widen(e0), w1 = widen(e1), w2 = widen(e2), w3 = widen(e3);
-    J[0][c] = c < 4 ? J[0][c] + w0 : w0;
-    J[1][c] = c < 4 ? J[1][c] + w1 : w1;
+    if (c >= 2) { // (a shift on the last plane has no field-induced part)
+      J[0][c] = c < 4 ? J[0][c] + w0 : w0;
+      J[1][c] = c < 4 ? J[1][c] + w1 : w1;
+    }
     J[2][c] = c >= 2 && c < 4 ? J[2][c] + w2 : w2;
     J[3][c] = c >= 2 && c < 4 ? J[3][c] + w3 : w3;
     if (time) J5[c] = (double)R3[c];
@@ -1073,7 +1072,9 @@ __device__ __forceinline__ void updateState(LT &L, const Params &P, const PlaneD
 #pragma unroll
   for (int r = 0; r < 3; ++r) L.pos[r] = fma(pl.U[r], loc0, fma(pl.V[r], loc1, pl.c[r]));
   double cP, sP, cT, sT;
-  if (!(fabs(dphi) <= 0.02) || !(fabs(dth) <= 0.02) || !(t.sT > 1e-6)) {
+  // (comparisons as integers: 0.02 and 1e-6 by their bits; NaN compares large)
+  if (akey(dphi) > 0x3f947ae147ae147bLL || akey(dth) > 0x3f947ae147ae147bLL ||
+      !(okey(t.sT) > 0x3eb0c6f7a0b5ed8dLL) || akey(t.sT) > 0x7ff0000000000000LL) {
     sincos(atan2(t.sP, t.cP) + dphi, &sP, &cP);
     sincos(atan2(t.sT, t.cT) + dth, &sT, &cT);
   } else {
@@ -1159,6 +1160,12 @@ __device__ __forceinline__ Gain gain(double S00, double S01, double S11, double 
   g.chi2 = fma(r0, e0, rp * g.e1);
   g.e0 = fma(-g.l, g.e1, e0);
   return g;
+}
+
+// chi2 above the cut, if there is one (as integers; NaN is no outlier)
+__device__ __forceinline__ bool isOutlier(const Params &P, double chi2) {
+  const long long k = okey(chi2);
+  return P.cutKey >= 0 && k > P.cutKey && k <= 0x7ff0000000000000LL;
 }
 
 // ---------------------------------------------------------------------------
@@ -1277,7 +1284,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT, H> &L, const Params
       a11 = fma(h1[i], w1[i], a11);
     }
     const Gain g = gain(a00 + v00, a01 + v01, a11 + v11, m0 - x0, m1 - x1);
-    outlier = (P.outlierCut > 0. && g.chi2 > P.outlierCut);
+    outlier = isOutlier(P, g.chi2);
     if (!outlier) {
       double dl[5];
 #pragma unroll
@@ -1399,7 +1406,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT, H> &L, const Params
       }
     }
     const Gain g = gain(C[0] + v00, C[1] + v01, C[u5(1, 1)] + v11, m0 - x0, m1 - x1);
-    outlier = (P.outlierCut > 0. && g.chi2 > P.outlierCut);
+    outlier = isOutlier(P, g.chi2);
     if (!outlier) {
       double w0[5], w1[5], a0[5], a1[5], dl[5];
 #pragma unroll
@@ -1791,18 +1798,15 @@ __device__ __forceinline__ void initFit(FitLane<FORM, MAT, H> &L, const Params &
   }
   // momentum and position on the line (coordinate_transformations.hpp:45-76,
   // LineSurface.ipp:184-198)
-  const double pabs = fabs(1. / sp[4]);
   double sph, cph, sth, cth;
   sincos(sp[2], &sph, &cph);
   sincos(sp[3], &sth, &cth);
-  const double mom[3] = {pabs * sth * cph, pabs * sth * sph, pabs * cth};
-  const double rad0 = -mom[1], rad1 = mom[0]; // (0,0,1) x mom
-  const double rn = sqrt(rad0 * rad0 + rad1 * rad1);
-  const double pg[3] = {per[0] + sp[0] * (rad0 / rn), per[1] + sp[0] * (rad1 / rn),
-                        (sp[1] + per[2]) + sp[0] * (0. / rn)};
-  const double pn = sqrt(mom[0] * mom[0] + mom[1] * mom[1] + mom[2] * mom[2]);
-  const double ip = 1. / pn;
-  const double dg[3] = {mom[0] * ip, mom[1] * ip, mom[2] * ip};
+  const double ip = fabs(sp[4]);
+  const double dg[3] = {sth * cph, sth * sph, cth};
+  // the radial axis (0,0,1) x d / |...|, undefined (NaN) along the line
+  const double sg = sth > 0. ? 1. : (sth < 0. ? -1. : __longlong_as_double(0x7ff8000000000000LL));
+  const double r = sp[0] * sg;
+  const double pg[3] = {fma(-r, sph, per[0]), fma(r, cph, per[1]), (sp[1] + per[2]) + 0. * r};
   toFrame<LT>(P, pg, L.pos);
   toFrame<LT>(P, dg, L.dir);
   L.q = (sp[4] > 0) ? 1. : -1.;

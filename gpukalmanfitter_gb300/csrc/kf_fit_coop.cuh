@@ -220,7 +220,7 @@ __device__ __forceinline__ void filterHit(CoopLane<FORM> &L, const Params &P, co
     a11 = fma(h1[i], w1[i], a11);
   }
   const Gain g = gain(a00 + v00, a01 + v01, a11 + v11, m0 - x0, m1 - x1);
-  const bool outlier = (P.outlierCut > 0. && g.chi2 > P.outlierCut);
+  const bool outlier = isOutlier(P, g.chi2);
   Trig tn = tr;
   if (!outlier) {
     double dl[5], dlc = 0., w0c = 0., w1c = 0.;
