@@ -560,6 +560,41 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
   L.rkSteps++;
 }
 
+// error estimate of a trial step in FP64 (EigenStepper.ipp:243-269); one
+// rejected lane makes its whole warp wait for it
+__device__ __forceinline__ double trialError(const FieldD &F, const double pos[3], const double dir[3],
+                                             double qop, double h) {
+  if (F.kind == KF_FIELD_CONSTANT) {
+    kfa::PolyStep w;
+    kfa::polyTrialFwd(dir, qop, h, F.B, w);
+    return w.err;
+  }
+  double b[3], k1[3], k2[3], k3[3], k4[3], t[3];
+  const double hh = 0.5 * h, h2 = h * h;
+  fieldScaled(F, pos, qop, b);
+  cross3(dir, b, k1);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) t[i] = fma(0.125 * h2, k1[i], fma(hh, dir[i], pos[i]));
+  fieldScaled(F, t, qop, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) t[i] = fma(hh, k1[i], dir[i]);
+  cross3(t, b, k2);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) t[i] = fma(hh, k2[i], dir[i]);
+  cross3(t, b, k3);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) t[i] = fma(0.5 * h2, k3[i], fma(h, dir[i], pos[i]));
+  fieldScaled(F, t, qop, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) t[i] = fma(h, k3[i], dir[i]);
+  cross3(t, b, k4);
+  double e = 0.;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) e += fabs(k1[i] - k2[i] - k3[i] + k4[i]);
+  e *= h2;
+  return (e < 1e-20) ? 1e-20 : e;
+}
+
 // Mixed form: FP32 stage offsets from an FP64 k1, FP32 transport
 // (rkTrialDelta, applyTransportOffsets), FP64 position and direction.  The
 // FP32 estimate accepts below 99 % of the tolerance; otherwise the FP64 trial
@@ -584,9 +619,7 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMix
     hf = narrow(h);
     const float errf = rkTrialDelta(P.field, posf, res, dirf, qopf, hf, S);
     if (errf <= P.tolLoF) break;
-    RkStages<double> sd;
-    rkFirst<double>(P.field, L.pos, L.dir, L.qop, sd);
-    const double err = rkTrial<double>(P.field, L.pos, L.dir, L.qop, h, sd);
+    const double err = trialError(P.field, L.pos, L.dir, L.qop, h);
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) return;
   }
