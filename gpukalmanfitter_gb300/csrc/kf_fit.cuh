@@ -450,16 +450,39 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
   const float4 v001 = __ldg(g + nxy), v101 = __ldg(g + nxy + 1), v011 = __ldg(g + nxy + nx),
                v111 = __ldg(g + nxy + nx + 1);
   const double s = F.scale * qop;
+  // The differences of neighbours along x are taken in FP32, where they are
+  // exact for values within a factor of 2 of each other (Sterbenz), as almost
+  // all are; TwoSum's error term tells, and any inexact one sends the lookup
+  // through FP64 differences: 12 of 42 FP64 instructions a lookup less.
+  float off = 0.f;
+  auto dif = [&](float a, float b) {
+    const float e = __fsub_rn(b, a), t = __fsub_rn(e, b);
+    off = fmaxf(off, fabsf(__fsub_rn(__fsub_rn(b, __fsub_rn(e, t)), __fadd_rn(a, t))));
+    return widen(e);
+  };
+  auto mix = [](double a, double b, double w) { return fma(w, b - a, a); };
   auto tri = [&](float a000, float a100, float a010, float a110, float a001, float a101,
                  float a011, float a111) {
-    auto mix = [](double a, double b, double w) { return fma(w, b - a, a); };
-    const double c0 = mix(mix(widen(a000), widen(a100), f[0]), mix(widen(a010), widen(a110), f[0]), f[1]);
-    const double c1 = mix(mix(widen(a001), widen(a101), f[0]), mix(widen(a011), widen(a111), f[0]), f[1]);
-    return mix(c0, c1, f[2]) * s;
+    const double c00 = fma(f[0], dif(a000, a100), widen(a000));
+    const double c10 = fma(f[0], dif(a010, a110), widen(a010));
+    const double c01 = fma(f[0], dif(a001, a101), widen(a001));
+    const double c11 = fma(f[0], dif(a011, a111), widen(a011));
+    return mix(mix(c00, c10, f[1]), mix(c01, c11, f[1]), f[2]) * s;
   };
   B[0] = tri(v000.x, v100.x, v010.x, v110.x, v001.x, v101.x, v011.x, v111.x);
   B[1] = tri(v000.y, v100.y, v010.y, v110.y, v001.y, v101.y, v011.y, v111.y);
   B[2] = tri(v000.z, v100.z, v010.z, v110.z, v001.z, v101.z, v011.z, v111.z);
+  if (!(off == 0.f)) {
+    auto tri64 = [&](float a000, float a100, float a010, float a110, float a001, float a101,
+                     float a011, float a111) {
+      const double c00 = mix(widen(a000), widen(a100), f[0]), c10 = mix(widen(a010), widen(a110), f[0]);
+      const double c01 = mix(widen(a001), widen(a101), f[0]), c11 = mix(widen(a011), widen(a111), f[0]);
+      return mix(mix(c00, c10, f[1]), mix(c01, c11, f[1]), f[2]) * s;
+    };
+    B[0] = tri64(v000.x, v100.x, v010.x, v110.x, v001.x, v101.x, v011.x, v111.x);
+    B[1] = tri64(v000.y, v100.y, v010.y, v110.y, v001.y, v101.y, v011.y, v111.y);
+    B[2] = tri64(v000.z, v100.z, v010.z, v110.z, v001.z, v101.z, v011.z, v111.z);
+  }
 }
 
 // Field map, FP64 stage by stage (EigenStepper.ipp:243-332), with q/p folded
@@ -478,8 +501,7 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
   cross3(L.dir, b1, k1);
   for (;;) {
     L.rkTrials++;
-    const double hh = 0.5 * h, h2 = h * h;
-    const double h8 = 0.25 * hh * h;
+    const double hh = 0.5 * h, h22 = hh * h, h8 = 0.25 * h22;
 #pragma unroll
     for (int i = 0; i < 3; ++i) t[i] = fma(h8, k1[i], fma(hh, L.dir[i], L.pos[i]));
     fieldScaled(P.field, t, L.qop, b2);
@@ -489,18 +511,28 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
 #pragma unroll
     for (int i = 0; i < 3; ++i) t[i] = fma(hh, k2[i], L.dir[i]);
     cross3(t, b2, k3);
-    const double h22 = hh * h;
 #pragma unroll
     for (int i = 0; i < 3; ++i) t[i] = fma(h22, k3[i], fma(h, L.dir[i], L.pos[i]));
     fieldScaled(P.field, t, L.qop, b3);
 #pragma unroll
     for (int i = 0; i < 3; ++i) t[i] = fma(h, k3[i], L.dir[i]);
     cross3(t, b3, k4);
+    // in FP32 first: the estimate with a bound of its rounding (four values
+    // of |k| at 2^-24 each and the sums': below 1e-6 |k|) decides unless it
+    // comes near the tolerance
+    {
+      const float hf = narrow(h);
+      float e = 0.f;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const float a = narrow(k1[i]), b = narrow(k2[i]), c = narrow(k3[i]), d = narrow(k4[i]);
+        e += fabsf((a - b) + (d - c)) + 1e-6f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d));
+      }
+      if (hf * hf * e <= P.tolAcceptF) break;
+    }
     const double d0 = k1[0] - k2[0] - k3[0] + k4[0], d1 = k1[1] - k2[1] - k3[1] + k4[1],
                  d2 = k1[2] - k2[2] - k3[2] + k4[2];
-    const float hf = (float)h;
-    if (hf * hf * (fabsf((float)d0) + fabsf((float)d1) + fabsf((float)d2)) <= P.tolAcceptF) break;
-    const double e = h2 * (fabs(d0) + fabs(d1) + fabs(d2));
+    const double e = h * h * (fabs(d0) + fabs(d1) + fabs(d2));
     const double err = (e < 1e-20) ? 1e-20 : e;
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) return;
