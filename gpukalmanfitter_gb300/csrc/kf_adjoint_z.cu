@@ -11,8 +11,8 @@
 //
 // A. forward: the fit's lane, whose hook stores per state (F, C0, D before the
 //    update, the predicted state, the leg's transport scalars; 70 words) and
-//    tapes the RK steps and step constraints (13 and 2 words) and the
-//    Jacobian per hit;
+//    tapes the RK steps and step constraints (13 and 2 words) and per hit the
+//    Jacobian, C0 h and the gain (36);
 // B. chi2 and sum of dchi2/dE over the states;
 // C. backwards over the tape: reverseStep (the RK step and its transport
 //    scalars) and reverseEvent (update, F <- J F, Jacobian from the leg).
@@ -48,8 +48,11 @@ enum {
   zTr = 61,   // trigonometry of the predicted direction
   zTn = 65,   // ... and of the filtered one
   zStep = 69, // a step since the last surface
-  zWords = 70
+  zRho = 70,  // 2 V^-1 rho (written by chi2States)
+  zWords = 72
 };
+// a hit's tape record: J (20), W = C0 [h0 h1] (10), the gain's l, i0, i1, e0, e1
+enum { tJ = 0, tW = 20, tGain = 30, tWords = 35 };
 static_assert(zWords <= 2 * kStateStride, "state record");
 
 struct ZHook {
@@ -158,6 +161,18 @@ struct ZHook {
     for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int c = 0; c < 5; ++c) put(J[r][c]);
+  }
+  __device__ __forceinline__ void update(const double (&w0)[5], const double (&w1)[5], const Gain &g) {
+    if (!rec) return;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) put(w0[c]);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) put(w1[c]);
+    put(g.l);
+    put(g.i0);
+    put(g.i1);
+    put(g.e0);
+    put(g.e1);
   }
   __device__ __forceinline__ void eventEnd(bool outlier, const Trig &tn) {
     info[(int64_t)state * n] = plane | (outlier ? 256 : 0);
@@ -352,50 +367,24 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
     }
 #pragma unroll
     for (int e = 0; e < 15; ++e) C[e] = rec(s, zC + e);
-    const double *mp = P.meas + (size_t)k * 5 * P.stride + i;
-    const double m0 = mp[0], m1 = mp[P.stride], v00 = mp[2 * P.stride], v01 = mp[3 * P.stride],
-                 v11 = mp[4 * P.stride];
     // chi2's own term
-    double p0, p1;
-    {
-      double E[5], f0 = m0 - x0, f1 = m1 - x1;
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        E[c] = L.D(c) - rec(s, zD + c);
-        f0 = fma(-h0[c], E[c], f0);
-        f1 = fma(-h1[c], E[c], f1);
-      }
-      const double id = 2. * rcpFast(v00 * v11 - v01 * v01);
-      p0 = (v11 * f0 - v01 * f1) * id;
-      p1 = (v00 * f1 - v01 * f0) * id;
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        L.F(0, c) = fma(-p0, E[c], L.F(0, c));
-        L.F(1, c) = fma(-p1, E[c], L.F(1, c));
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < 5; ++a) {
-      double e = C[u5(a, 0)] * h0[0], f = C[u5(a, 0)] * h1[0];
-#pragma unroll
-      for (int j = 1; j < 5; ++j) {
-        e = fma(C[u5(a, j)], h0[j], e);
-        f = fma(C[u5(a, j)], h1[j], f);
-      }
-      w0[a] = e;
-      w1[a] = f;
-    }
-    double a00 = 0., a01 = 0., a11 = 0.;
+    const double p0 = rec(s, zRho), p1 = rec(s, zRho + 1);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-      a00 = fma(h0[c], w0[c], a00);
-      a01 = fma(h1[c], w0[c], a01);
-      a11 = fma(h1[c], w1[c], a11);
+      const double E = L.D(c) - rec(s, zD + c);
+      L.F(0, c) = fma(-p0, E, L.F(0, c));
+      L.F(1, c) = fma(-p1, E, L.F(1, c));
+      w0[c] = Jt[tW + c];
+      w1[c] = Jt[tW + 5 + c];
     }
-    const Gain g = gain(a00 + v00, a01 + v01, a11 + v11, m0 - x0, m1 - x1);
-    double dl[5];
+    const Gain g = {Jt[tGain], Jt[tGain + 1], Jt[tGain + 2], Jt[tGain + 3], Jt[tGain + 4], 0.};
+    double dl[5], D0 = 0., D1 = 0.; // h . dl: the shift of the predicted position
 #pragma unroll
-    for (int c = 0; c < 5; ++c) dl[c] = fma(w0[c], g.e0, w1[c] * g.e1);
+    for (int c = 0; c < 5; ++c) {
+      dl[c] = fma(w0[c], g.e0, w1[c] * g.e1);
+      D0 = fma(h0[c], dl[c], D0);
+      D1 = fma(h1[c], dl[c], D1);
+    }
     // the stepper's new direction and position
     double ph1, th1, X0b, X1b;
     {
@@ -404,7 +393,7 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
       th1 = tn.cT * (tn.cP * R.dir[0] + tn.sP * R.dir[1]) - tn.sT * R.dir[2];
       phb += ph1;
       thb += th1;
-      const double X0 = x0 + fma(a00, g.e0, a01 * g.e1), X1 = x1 + fma(a01, g.e0, a11 * g.e1);
+      const double X0 = x0 + D0, X1 = x1 + D1;
       X0b = dot3(pl.U, R.pos);
       X1b = dot3(pl.V, R.pos);
 #pragma unroll
@@ -512,7 +501,7 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
     for (int r = 0; r < 4; ++r) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        J[r][c] = Jt[5 * r + c];
+        J[r][c] = Jt[tJ + 5 * r + c];
         Jb[r][c] = 0.;
       }
       Jb[r][4] = L.F(r, 4);
@@ -714,7 +703,8 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
   R.dir[2] += thb * f1[2];
 }
 
-// chi2 of a track with ns states, and with grad the sum of dchi2/dE into Ct
+// chi2 of a track with ns states, the sum of dchi2/dE into Ct, and with grad
+// each state's 2 V^-1 rho into its record
 __device__ double chi2States(ZLane &L, const Params &P, const AdjParams &A, int64_t u, int64_t i,
                              int ns) {
   const int64_t n = P.n;
@@ -737,6 +727,11 @@ __device__ double chi2States(ZLane &L, const Params &P, const AdjParams &A, int6
     const double id = rcpFast(v00 * v11 - v01 * v01);
     const double w0 = (v11 * f0 - v01 * f1) * id, w1 = (v00 * f1 - v01 * f0) * id;
     chi2 += f0 * w0 + f1 * w1;
+    if (A.grad) {
+      double *rb = A.stateBar + ((int64_t)s * kStateStride + zRho - kStateStride) * n + u;
+      rb[0] = 2. * w0;
+      rb[n] = 2. * w1;
+    }
 #pragma unroll
     for (int c = 0; c < 5; ++c) G[c] -= 2. * (w0 * h0[c] + w1 * h1[c]);
   }

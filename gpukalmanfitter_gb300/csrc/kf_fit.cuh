@@ -1350,6 +1350,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT, H> &L, const Params
     }
     const Gain g = gain(a00 + v00, a01 + v01, a11 + v11, m0 - x0, m1 - x1);
     outlier = isOutlier(P, g.chi2);
+    if constexpr (LT::kTape) L.hook.update(w0, w1, g);
     if (!outlier) {
       double dl[5];
 #pragma unroll
