@@ -261,6 +261,8 @@ Staging stagingLayout(int64_t n, int32_t S, bool withSmoothed, const kf_config_t
 cudaError_t copyRows(void *dst, size_t dpitchElems, const void *src, size_t spitchElems,
                      size_t elem, size_t n, size_t rows, cudaMemcpyKind kind, cudaStream_t s) {
   if (!rows || !n) return cudaSuccess;
+  // contiguous on both sides (an unchunked call without padding): one row
+  if (dpitchElems == n && spitchElems == n) return cudaMemcpyAsync(dst, src, rows * n * elem, kind, s);
   return cudaMemcpy2DAsync(dst, dpitchElems * elem, src, spitchElems * elem, n * elem, rows, kind, s);
 }
 
