@@ -434,15 +434,14 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
     // rounding down
     const double gr = fma(p[a], F.invw[a], F.off[a]);
     const double t = __dadd_rd(gr, 6755399441055744.);
+    // clamped to the grid (outside it the edge cell extends): the low word is
+    // the index where the high word says so, and beyond 2^31 only the sign counts
     int i = __double2loint(t);
-    double fi = t - 6755399441055744.;
-    const int lim = F.n[a] - 2;
-    if (i < 0 || i > lim || !(fabs(gr) < 1e9)) { // outside the grid: the edge cell's extension
-      i = gr > 0. ? lim : 0;
-      fi = (double)i;
-    }
+    const int hi = __double2hiint(t);
+    if (hi != 0x43380000 || i < 0) i = hi == 0x4337ffff || __double2hiint(gr) < 0 ? 0 : F.n[a] - 2;
+    i = min(i, F.n[a] - 2);
     idx[a] = i;
-    f[a] = gr - fi;
+    f[a] = gr - (__hiloint2double(0x43380000, i) - 6755399441055744.);
   }
   const size_t nx = F.n[0], nxy = (size_t)F.n[0] * F.n[1];
   const float4 *g = F.grid + ((size_t)idx[2] * nxy + (size_t)idx[1] * nx + idx[0]);
@@ -521,11 +520,12 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
     // of |k| at 2^-24 each and the sums': below 1e-6 |k|) decides unless it
     // comes near the tolerance
     {
-      const float hf = narrow(h);
+      const float hf = narrow<true>(h);
       float e = 0.f;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        const float a = narrow(k1[i]), b = narrow(k2[i]), c = narrow(k3[i]), d = narrow(k4[i]);
+        const float a = narrow<true>(k1[i]), b = narrow<true>(k2[i]), c = narrow<true>(k3[i]),
+                    d = narrow<true>(k4[i]);
         e += fabsf((a - b) + (d - c)) + 1e-6f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d));
       }
       if (hf * hf * e <= P.tolAcceptF) break;
