@@ -13,6 +13,12 @@
 // steps there would run with the others idle (tracks with 10 % holes: 1.24
 // instead of 1.45 times the warp instructions of a track without divergence).
 //
+// With P.align (the mixed form's queue) the eight warps of a block run each
+// event together: the mixed kernel's code is larger than the instruction
+// caches near the schedulers, and a third of its stalls were instruction
+// fetches; warps in step share them (1M map tracks 44.8 -> 40.2 ms; stepping
+// together too gave no more, and the FP64 forms, whose pipe is full, lose 1 %).
+//
 // The block size is a run-time value: an instantiation is a register budget,
 // so that every shape of one budget, queue or not, gives the same bits.
 #pragma once
@@ -23,16 +29,19 @@ namespace kfd {
 
 // Fit the tracks i (inputs/outputs) with workspace columns w of one warp;
 // i < 0 marks an idle lane.  All 32 lanes must call it together.
+// align: the block's warps run their events together (all must call).
 template <int FORM, bool MAT, class H = NoHook>
-__device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64_t i, int64_t w) {
+__device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64_t i, int64_t w,
+                                        bool align = false) {
   FitLane<FORM, MAT, H> L;
   initFit(L, P, sp, i, w);
   for (;;) {
     if (!L.parked && L.pc != PC_DONE) advance(L, P, sp);
     const bool waiting = L.parked || L.pc == PC_DONE;
     if (__all_sync(0xffffffffu, waiting)) {
+      if (align) __syncthreads();
       if (L.parked) runEvent(L, P, sp);
-      if (__all_sync(0xffffffffu, L.pc == PC_DONE)) break;
+      if (align ? __syncthreads_and(L.pc == PC_DONE) : __all_sync(0xffffffffu, L.pc == PC_DONE)) break;
     }
   }
   if (i >= 0 && i < P.n && (threadIdx.x & (H::kGroup - 1)) == 0) {
@@ -55,22 +64,29 @@ __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ 
   for (int k = threadIdx.x; k < P.nSurf; k += blockDim.x) sp[k] = P.planes[k];
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const bool queue = P.queueCounter != nullptr;
+  const bool queue = P.queueCounter != nullptr, align = P.align != 0;
   const int lanes = P.lanes;
+  __shared__ int claim;
   for (;;) {
     int64_t base;
-    if (queue) {
+    if (align) { // the block claims its next tracks together
+      __syncthreads();
+      if (threadIdx.x == 0) claim = atomicAdd(P.queueCounter, (int)blockDim.x);
+      __syncthreads();
+      if (claim >= P.n) break;
+      base = claim + (threadIdx.x & ~31);
+    } else if (queue) {
       int b = 0;
       if (lane == 0) b = atomicAdd(P.queueCounter, lanes);
       base = (int64_t)__shfl_sync(0xffffffffu, b, 0);
     } else {
       base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lanes;
     }
-    if (base >= P.n) break;
+    if (!align && base >= P.n) break;
     const int64_t q = base + lane;
     const bool own = lane < lanes && q < P.n;
     const int64_t i = own ? (P.perm ? (int64_t)P.perm[q] : q) : -1;
-    fitWarp<FORM, MAT>(P, sp, i, own ? q : 0);
+    fitWarp<FORM, MAT>(P, sp, i, own ? q : 0, align);
     if (!queue) break;
   }
 }

@@ -48,7 +48,7 @@ const Shape kShapes[] = {
     {128, 4, &kBudget128}, {64, 8, &kBudget128},  {256, 2, &kBudget128}, {128, 5, &kBudget96},
 };
 // one-warp blocks spread over the SMs most evenly
-constexpr int kDefaultBlock = 32;
+constexpr int kDefaultBlock = 32, kQueueBlock = 256;
 
 } // namespace
 
@@ -174,7 +174,10 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   }
   if (sp.queue) P.queueCounter = q.counter;
   const Budget *b = P.materialEffects ? &kMaterial : shape->budget;
-  const int block = asked ? shape->bs : kDefaultBlock;
+  // with a queue one block of 8 warps an SM (2 % over one-warp blocks: warps
+  // that start together share instruction fetches)
+  const int block = asked ? shape->bs : sp.queue ? kQueueBlock : kDefaultBlock;
+  P.align = !asked && sp.queue && mixed && !P.materialEffects;
   if (mixed) {
     e = b->mixed(P, block, s);
   } else if (!uniform) {
