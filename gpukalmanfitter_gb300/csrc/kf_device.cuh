@@ -285,9 +285,12 @@ static __device__ __noinline__ void getFieldFFRZ(const FieldD &F, const float p[
 // cell-sized number instead of the position's (6e-5 mm at 1 m, which moves
 // the fitted d0 by up to 1e-5 of its resolution on the 30-plane map
 // telescope).
+//
+// MAP 0: a uniform field, 1: a map, -1: as F.kind says
+template <int MAP = -1>
 __device__ __forceinline__ void getFieldFF(const FieldD &F, const float at[3],
                                            const float inc[3], kff::ff B[3]) {
-  if (F.kind == KF_FIELD_CONSTANT) {
+  if (MAP == 0 || (MAP < 0 && F.kind == KF_FIELD_CONSTANT)) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) B[a] = {F.Bf[a], F.Blo[a]};
     return;
@@ -666,9 +669,10 @@ struct StagesDelta {
 };
 
 // posf: the step's start rounded to FP32, res: that rounding's residual
+template <int MAP = -1>
 __device__ __forceinline__ void rkFirstDelta(const FieldD &F, const float posf[3], const float res[3],
                                              const double dir[3], double qop, StagesDelta &S) {
-  getFieldFF(F, posf, res, S.Bf);
+  getFieldFF<MAP>(F, posf, res, S.Bf);
   double B[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -686,6 +690,7 @@ __device__ __forceinline__ void rkFirstDelta(const FieldD &F, const float posf[3
 
 // tryRungeKuttaStep (EigenStepper.ipp:243-269) as FP32 offsets from k1; the
 // trial positions (pos + res + increment) only locate the field
+template <int MAP = -1>
 __device__ __forceinline__ float rkTrialDelta(const FieldD &F, const float pos[3], const float res[3],
                                               const float dir[3], float q, float h, StagesDelta &S) {
   const float h2 = h * h, half_h = h * 0.5f;
@@ -693,7 +698,7 @@ __device__ __forceinline__ float rkTrialDelta(const FieldD &F, const float pos[3
   kff::ff B[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) p1[i] = res[i] + half_h * dir[i] + (h2 * 0.125f) * S.s.k1[i];
-  getFieldFF(F, pos, p1, B);
+  getFieldFF<MAP>(F, pos, p1, B);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     S.s.Bm[i] = B[i].hi;
@@ -714,7 +719,7 @@ __device__ __forceinline__ float rkTrialDelta(const FieldD &F, const float pos[3
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i) p1[i] = res[i] + h * dir[i] + (h2 * 0.5f) * S.s.k3[i];
-  getFieldFF(F, pos, p1, B);
+  getFieldFF<MAP>(F, pos, p1, B);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     S.s.Bl[i] = B[i].hi;

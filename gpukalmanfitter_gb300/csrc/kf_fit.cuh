@@ -54,8 +54,11 @@ namespace kfd {
 
 // kUniform64: FP64, uniform field along +-z; kUniformAny: in any other
 // direction (planes rotated into the field's frame); kGrid64: FP64, field
-// map; kMixed: mixed precision, any field
-enum FitForm { kUniform64 = 0, kGrid64 = 1, kMixed = 2, kUniformAny = 3 };
+// map; kMixed: mixed precision, field map; kMixedUniform: mixed precision,
+// uniform field (without the lookups' code: the mixed kernels wait for
+// instruction fetches)
+enum FitForm { kUniform64 = 0, kGrid64 = 1, kMixed = 2, kUniformAny = 3, kMixedUniform = 4 };
+__host__ __device__ constexpr bool isMixed(int form) { return form == kMixed || form == kMixedUniform; }
 __host__ __device__ constexpr bool isUniform(int form) { return form == kUniform64 || form == kUniformAny; }
 
 // ---- FP64 reciprocal and reciprocal square root -----------------------------
@@ -113,8 +116,10 @@ template <> struct LegState<kGrid64> {
 // mixed: FP32 transport blocks as offsets from the straight line
 // (applyTransportOffsets)
 template <> struct LegState<kMixed> {};
+template <> struct LegState<kMixedUniform> {};
 template <> struct LegState<kUniform64, 8> : LegState<kUniform64> {};
 template <> struct LegState<kMixed, 8> {};
+template <> struct LegState<kMixedUniform, 8> {};
 // each lane of a group carries its own column (2: phi, 3: theta, 4: q/p)
 template <> struct LegState<kGrid64, 8> {
   double p[3], v[3], s, k4[3];
@@ -127,7 +132,7 @@ struct MixedBlocks {
 };
 
 template <int FORM, bool MAT_, class H_ = NoHook>
-struct FitLane : std::conditional<FORM == kMixed, MixedBlocks, NoBlocks>::type {
+struct FitLane : std::conditional<isMixed(FORM), MixedBlocks, NoBlocks>::type {
   static constexpr int kForm = FORM;
   static constexpr bool kMat = MAT_;
   static constexpr bool kTape = H_::kTape;
@@ -229,13 +234,13 @@ template <class LT> __device__ __forceinline__ double *recPtr(const Params &P, c
 template <class LT>
 __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, bool time) {
   L.qop = L.q * ip;
-  if constexpr (LT::kForm == kMixed) L.qopf = narrow(L.qop);
+  if constexpr (isMixed(LT::kForm)) L.qopf = narrow(L.qop);
   if (time) {
     const double x = P.mass * ip, a = fma(x, x, 1.);
     const double y = rsqrtFast(a);
     L.dtds = a * y;
     L.d37 = P.mass * P.mass * L.qop * y;
-    if constexpr (LT::kForm == kMixed) L.d37f = (float)L.d37;
+    if constexpr (isMixed(LT::kForm)) L.d37f = (float)L.d37;
   }
 }
 
@@ -594,13 +599,15 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
 
 // error estimate of a trial step in FP64 (EigenStepper.ipp:243-269); one
 // rejected lane makes its whole warp wait for it
-__device__ __forceinline__ double trialError(const FieldD &F, const double pos[3], const double dir[3],
-                                             double qop, double h) {
-  if (F.kind == KF_FIELD_CONSTANT) {
-    kfa::PolyStep w;
-    kfa::polyTrialFwd(dir, qop, h, F.B, w);
-    return w.err;
-  }
+__device__ __forceinline__ double trialErrorUniform(const FieldD &F, const double dir[3], double qop,
+                                                    double h) {
+  kfa::PolyStep w;
+  kfa::polyTrialFwd(dir, qop, h, F.B, w);
+  return w.err;
+}
+static __device__ __noinline__ double trialError(const FieldD &F, double p0, double p1, double p2,
+                                                 double d0, double d1, double d2, double qop, double h) {
+  const double pos[3] = {p0, p1, p2}, dir[3] = {d0, d1, d2};
   double b[3], k1[3], k2[3], k3[3], k4[3], t[3];
   const double hh = 0.5 * h, h2 = h * h;
   fieldScaled(F, pos, qop, b);
@@ -636,7 +643,10 @@ __device__ __forceinline__ double trialError(const FieldD &F, const double pos[3
 // (the RK partition of the path) would drift from the FP64 fit's by ~3e-6,
 // so that a later decision near the tolerance could go the other way (1e-4 of
 // the perigee's resolution on a few tracks in 1e6).
-template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMixed, MAT, H> &L, const Params &P) {
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ typename std::enable_if<isMixed(FORM)>::type
+rkStep(FitLane<FORM, MAT, H> &L, const Params &P) {
+  constexpr int kMap = FORM == kMixed ? 1 : 0;
   long nTrials = 0;
   double h = ssValue(L);
   const float qopf = L.qopf;
@@ -645,13 +655,16 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kMix
   for (int i = 0; i < 3; ++i) split(L.pos[i], posf[i], res[i]);
   const float dirf[3] = {narrow(L.dir[0]), narrow(L.dir[1]), narrow(L.dir[2])};
   StagesDelta S;
-  rkFirstDelta(P.field, posf, res, L.dir, L.qop, S);
+  rkFirstDelta<kMap>(P.field, posf, res, L.dir, L.qop, S);
   for (;;) {
     L.rkTrials++;
     hf = narrow(h);
-    const float errf = rkTrialDelta(P.field, posf, res, dirf, qopf, hf, S);
+    const float errf = rkTrialDelta<kMap>(P.field, posf, res, dirf, qopf, hf, S);
     if (errf <= P.tolLoF) break;
-    const double err = trialError(P.field, L.pos, L.dir, L.qop, h);
+    const double err = FORM == kMixed
+                           ? trialError(P.field, L.pos[0], L.pos[1], L.pos[2], L.dir[0], L.dir[1],
+                                        L.dir[2], L.qop, h)
+                           : trialErrorUniform(P.field, L.dir, L.qop, h);
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) return;
   }
@@ -740,7 +753,7 @@ __device__ __forceinline__ void lastAxes(const LT &L, const Params &P, const Pla
     // LineSurface::referenceFrame at the start direction (LineSurface.ipp:
     // 46-61); the mixed form rounds its start Jacobian to FP32
     double x[3] = {-tl.sP, tl.cP, 0.}, y[3] = {0., 0., 1.};
-    if (LT::kForm == kMixed) {
+    if (isMixed(LT::kForm)) {
       x[0] = (double)(float)x[0];
       x[1] = (double)(float)x[1];
     }
@@ -831,7 +844,7 @@ __device__ __forceinline__ void lastK4(const FitLane<kGrid64, MAT, H> &L, const 
   for (int i = 0; i < 3; ++i) k4[i] = L.g.k4[i];
 }
 template <int FORM, bool MAT, class H> __device__ __forceinline__ double legPath(const FitLane<FORM, MAT, H> &L) {
-  if constexpr (FORM == kMixed) return L.sTr;
+  if constexpr (isMixed(FORM)) return L.sTr;
   else return L.g.s;
 }
 
@@ -914,7 +927,8 @@ __device__ __forceinline__ void angleRows(const Params &P, const Trig &t, double
 
 // at a plane, FP64 forms; tr: trigonometry of the direction there
 template <int FORM, bool MAT, class H>
-__device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
+__device__ __forceinline__ typename std::enable_if<!isMixed(FORM)>::type
+boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
                                               const PlaneD *planes, const PlaneD &pl, bool time,
                                               Trig &tr, double (&J)[4][5], double (&J5)[5]) {
   using LT = FitLane<FORM, MAT, H>;
@@ -943,11 +957,12 @@ __device__ __forceinline__ void boundJacobian(const FitLane<FORM, MAT, H> &L, co
 // out accurate to FP32 rounding of those small terms (an FP32 J moves the
 // fitted perigee by up to 3e-6 of its resolution on the 30-plane map
 // telescope, mostly through the angle rows).
-template <bool MAT, class H>
-__device__ __forceinline__ void boundJacobian(const FitLane<kMixed, MAT, H> &L, const Params &P,
+template <int FORM, bool MAT, class H>
+__device__ __forceinline__ typename std::enable_if<isMixed(FORM)>::type
+boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
                                               const PlaneD *planes, const PlaneD &pl, bool time,
                                               Trig &tr, double (&J)[4][5], double (&J5)[5]) {
-  using LT = FitLane<kMixed, MAT, H>;
+  using LT = FitLane<FORM, MAT, H>;
   double invS;
   tr = trigOf(L.dir, invS);
   const Trig tl = trigLoad(L);
@@ -1631,7 +1646,7 @@ __device__ __forceinline__ void reachPerigee(FitLane<FORM, MAT, H> &L, const Par
 #pragma unroll
     for (int e = 0; e < 6; ++e) Ct[e] = L.Ct(e);
   }
-  if constexpr (FORM != kMixed) {
+  if constexpr (!isMixed(FORM)) {
     double invS;
     const Trig tr = trigOf(dg, invS);
     // X = z x d / |z x d|, Y = z (LineSurface::referenceFrame), the path

@@ -6,3 +6,4 @@
 KF_COOP_LAUNCHER(launchFitCoop_fp64_uniform, kfd::kUniform64)
 KF_COOP_LAUNCHER(launchFitCoop_fp64_grid, kfd::kGrid64)
 KF_COOP_LAUNCHER(launchFitCoop_mixed, kfd::kMixed)
+KF_COOP_LAUNCHER(launchFitCoop_mixed_uniform, kfd::kMixedUniform)

@@ -32,7 +32,7 @@ __device__ __forceinline__ void boundColumn(const CoopLane<FORM> &L, const Param
                                             const PlaneD *planes, const PlaneD &pl, int c, bool time,
                                             Trig &tr, double (&J)[4], double &J5) {
   using LT = CoopLane<FORM>;
-  if constexpr (FORM == kMixed) {
+  if constexpr (isMixed(FORM)) {
     double A[4][5], A5[5] = {0., 0., 0., 0., 0.};
     boundJacobian(L, P, planes, pl, time, tr, A, A5);
 #pragma unroll

@@ -5,3 +5,4 @@
 #include "kf_kernels.cuh"
 
 KF_FIT_LAUNCHER(launchFit_mixed_128, kfd::kMixed, false, 256, 2)
+KF_FIT_LAUNCHER(launchFit_mixed_uniform_128, kfd::kMixedUniform, false, 256, 2)

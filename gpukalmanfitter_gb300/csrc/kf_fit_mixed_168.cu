@@ -5,3 +5,4 @@
 #include "kf_kernels.cuh"
 
 KF_FIT_LAUNCHER(launchFit_mixed_168, kfd::kMixed, false, 128, 3)
+KF_FIT_LAUNCHER(launchFit_mixed_uniform_168, kfd::kMixedUniform, false, 128, 3)

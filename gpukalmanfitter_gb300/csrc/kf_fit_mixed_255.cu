@@ -5,3 +5,4 @@
 #include "kf_kernels.cuh"
 
 KF_FIT_LAUNCHER(launchFit_mixed_255, kfd::kMixed, false, 256, 1)
+KF_FIT_LAUNCHER(launchFit_mixed_uniform_255, kfd::kMixedUniform, false, 256, 1)

@@ -5,3 +5,4 @@
 #include "kf_kernels.cuh"
 
 KF_FIT_LAUNCHER(launchFit_mixed_96, kfd::kMixed, false, 128, 5)
+KF_FIT_LAUNCHER(launchFit_mixed_uniform_96, kfd::kMixedUniform, false, 128, 5)

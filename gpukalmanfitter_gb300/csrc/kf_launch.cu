@@ -9,7 +9,8 @@ using kfd::Params;
 #define KF_DECLARE_BUDGET(R)              \
   KF_DECLARE(launchFit_fp64_uniform_##R)  \
   KF_DECLARE(launchFit_fp64_grid_##R)     \
-  KF_DECLARE(launchFit_mixed_##R)
+  KF_DECLARE(launchFit_mixed_##R)         \
+  KF_DECLARE(launchFit_mixed_uniform_##R)
 KF_DECLARE_BUDGET(255)
 KF_DECLARE_BUDGET(168)
 KF_DECLARE_BUDGET(128)
@@ -19,9 +20,11 @@ KF_DECLARE(launchFitMaterial_fp64_any)
 KF_DECLARE(launchFitMaterial_fp64_uniform)
 KF_DECLARE(launchFitMaterial_fp64_grid)
 KF_DECLARE(launchFitMaterial_mixed)
+KF_DECLARE(launchFitMaterial_mixed_uniform)
 KF_DECLARE(launchFitCoop_fp64_uniform)
 KF_DECLARE(launchFitCoop_fp64_grid)
 KF_DECLARE(launchFitCoop_mixed)
+KF_DECLARE(launchFitCoop_mixed_uniform)
 KF_DECLARE(launchFitMaterialStates_fp64)
 KF_DECLARE(launchFitMaterialStates_mixed)
 
@@ -29,14 +32,16 @@ namespace {
 
 using Launch = cudaError_t (*)(const Params &, int, cudaStream_t);
 struct Budget {
-  Launch uniform, grid, mixed, anyField; // anyField: a uniform field off the z axis
+  Launch uniform, grid, mixedGrid, mixedUniform, anyField; // anyField: uniform, off the z axis
 };
 #define KF_BUDGET(R) \
-  {launchFit_fp64_uniform_##R, launchFit_fp64_grid_##R, launchFit_mixed_##R, launchFit_fp64_any}
+  {launchFit_fp64_uniform_##R, launchFit_fp64_grid_##R, launchFit_mixed_##R,  \
+   launchFit_mixed_uniform_##R, launchFit_fp64_any}
 const Budget kBudget255 = KF_BUDGET(255), kBudget168 = KF_BUDGET(168), kBudget128 = KF_BUDGET(128),
              kBudget96 = KF_BUDGET(96);
 const Budget kMaterial = {launchFitMaterial_fp64_uniform, launchFitMaterial_fp64_grid,
-                          launchFitMaterial_mixed, launchFitMaterial_fp64_any};
+                          launchFitMaterial_mixed, launchFitMaterial_mixed_uniform,
+                          launchFitMaterial_fp64_any};
 
 struct Shape {
   int bs, minb;
@@ -161,7 +166,8 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   if (!asked && !P.materialEffects && !P.oSmoothed && !offAxis && P.n <= kCoopMost * sms) {
     if (!mixed && uniform) toFieldFrame(P);
     P.lanes = (int)std::min<int64_t>(4, (P.n + kLeastWarps * sms - 1) / (kLeastWarps * sms));
-    e = (mixed ? launchFitCoop_mixed : uniform ? launchFitCoop_fp64_uniform : launchFitCoop_fp64_grid)(P, 0, s);
+    e = (mixed ? (uniform ? launchFitCoop_mixed_uniform : launchFitCoop_mixed)
+               : (uniform ? launchFitCoop_fp64_uniform : launchFitCoop_fp64_grid))(P, 0, s);
     return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
   }
   Spread sp = spread(P.n, sms);
@@ -179,7 +185,7 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   const int block = asked ? shape->bs : sp.queue ? kQueueBlock : kDefaultBlock;
   P.align = !asked && sp.queue && mixed && !P.materialEffects;
   if (mixed) {
-    e = b->mixed(P, block, s);
+    e = (uniform ? b->mixedUniform : b->mixedGrid)(P, block, s);
   } else if (!uniform) {
     e = b->grid(P, block, s);
   } else {
