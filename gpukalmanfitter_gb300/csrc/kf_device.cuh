@@ -127,19 +127,15 @@ __device__ __forceinline__ double widen(float f) {
 
 // FP64 to FP32, rounded to nearest even, on the integer pipe (a conversion
 // takes the FP64 pipe as long as an FMA); results below the least normal FP32
-// value come out as zero
-//
-// The predicated conversion for values beyond FP32 still takes the FP64 pipe
-// for some cycles; without it (INF: the two cases by selection) a kernel bound
-// by that pipe gains (field map FP64: 5.56 -> 5.33 ms for 50k tracks), one
-// near its integer limits loses (mixed: 44.8 -> 46.9 ms for 1M).
-template <bool INF = false> __device__ __forceinline__ float narrow(double d) {
+// value come out as zero, beyond the largest as infinity
+// (a predicated conversion in their place would take the FP64 pipe in every
+// call: 1M map tracks mixed 40.0 ms with it, 37.9 ms without)
+__device__ __forceinline__ float narrow(double d) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(d);
   const unsigned long long r = b + (0x0fffffffu + ((unsigned)(b >> 29) & 1u));
   const unsigned a = (unsigned)(r >> 32) & 0x7fffffffu;
-  if (!INF && a >= 0x47f00000u) return (float)d; // beyond FP32, infinite or NaN
   unsigned f = a < 0x38100000u ? 0u : ((unsigned)(r >> 29) + 0x40000000u) & 0x7fffffffu;
-  if (INF && a >= 0x47f00000u) f = a > 0x7ff00000u ? 0x7fffffffu : 0x7f800000u;
+  if (a >= 0x47f00000u) f = a > 0x7ff00000u ? 0x7fffffffu : 0x7f800000u; // NaN, beyond FP32
   return __uint_as_float(f | ((unsigned)(b >> 32) & 0x80000000u));
 }
 // d as narrow(d) and the FP32 rounding of the rest d - narrow(d), which is a
@@ -1192,21 +1188,12 @@ __device__ __forceinline__ void projectCov(Lane<R, H> &L, Transported<R> &X, con
 // direction, |p| and q/p as the stepper holds them.  The reference forms q/p
 // as charge / |p d| with p = |1 / (q/p)|; with |d| = 1 that is the stepper's
 // q/p to an ulp, without the three divisions and the square root.
-//
-// With absAngles == false the angles are given as offsets from the
-// direction's own angles, i.e. 0 (see filterHit).
 template <typename R, typename H>
-__device__ __forceinline__ void boundAngles(const Lane<R, H> &L, double out[6], double mom[3],
-                                            bool absAngles = true) {
+__device__ __forceinline__ void boundAngles(const Lane<R, H> &L, double out[6], double mom[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) mom[i] = L.p * L.dir[i];
-  if (absAngles) {
-    out[2] = atan2(L.dir[1], L.dir[0]);
-    out[3] = atan2(sqrt(L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1]), L.dir[2]);
-  } else {
-    out[2] = 0.;
-    out[3] = 0.;
-  }
+  out[2] = atan2(L.dir[1], L.dir[0]);
+  out[3] = atan2(sqrt(L.dir[0] * L.dir[0] + L.dir[1] * L.dir[1]), L.dir[2]);
   out[4] = L.qop;
   out[5] = L.t;
 }
@@ -1299,7 +1286,7 @@ __device__ __forceinline__ void transportCovD(Lane<R, H> &L, const double J[6][5
 // smoother take it in FP64.
 template <typename H>
 __device__ void boundStatePlaneMixed(Lane<float, H> &L, const PlaneD &pl, double out[6],
-                                     double Jst[25], bool absAngles) {
+                                     double Jst[25]) {
   const DirTrig<double> td = dirTrigD(L);
   const double s = L.sTr;
   const bool st = L.stepped;
@@ -1411,15 +1398,14 @@ __device__ void boundStatePlaneMixed(Lane<float, H> &L, const PlaneD &pl, double
   out[0] = pl.U[0] * d0 + pl.U[1] * d1 + pl.U[2] * d2;
   out[1] = pl.V[0] * d0 + pl.V[1] * d1 + pl.V[2] * d2;
   double mom[3];
-  boundAngles(L, out, mom, absAngles);
+  boundAngles(L, out, mom);
 }
 
 // boundState<PlaneSurface> (EigenStepper.ipp:516-540) incl. re-initialisation
 template <typename R, typename H>
-__device__ void boundStatePlane(Lane<R, H> &L, const PlaneD &pl, double out[6], double Jst[25],
-                                bool absAngles = true) {
+__device__ void boundStatePlane(Lane<R, H> &L, const PlaneD &pl, double out[6], double Jst[25]) {
   if constexpr (sizeof(R) == sizeof(float)) {
-    boundStatePlaneMixed(L, pl, out, Jst, absAngles);
+    boundStatePlaneMixed(L, pl, out, Jst);
     return;
   }
   Transported<R> X;
@@ -1443,7 +1429,7 @@ __device__ void boundStatePlane(Lane<R, H> &L, const PlaneD &pl, double out[6], 
   out[0] = pl.U[0] * d0 + pl.U[1] * d1 + pl.U[2] * d2;
   out[1] = pl.V[0] * d0 + pl.V[1] * d1 + pl.V[2] * d2;
   double mom[3];
-  boundAngles(L, out, mom, absAngles);
+  boundAngles(L, out, mom);
 }
 
 // boundState<LineSurface> towards the perigee line (axis z through `c`)
@@ -1515,29 +1501,15 @@ __device__ __forceinline__ void stepperUpdate(Lane<R, H> &L, const PlaneD &pl, c
 // <= 0.02: truncation below 1e-20 absolute).  The direction is scaled by
 // sin(theta_p) before its normalisation, which removes that division.  Larger
 // corrections, and directions within 1e-6 of the z axis, take stepperUpdate.
-//
-// pred and par may hold the angles as offsets from the predicted direction's
-// (absAngles == false); only their difference is used, and the rare
-// fallback restores the absolute filtered angles from the direction first.
 template <typename R, typename H>
 __device__ __forceinline__ void stepperUpdateFiltered(Lane<R, H> &L, const PlaneD &pl,
                                                       const double pred[6], const double par[6],
-                                                      const double cov[21], double mass,
-                                                      bool absAngles = true) {
+                                                      const double cov[21], double mass) {
   const double dphi = par[2] - pred[2], dth = par[3] - pred[3];
   const double dx = L.dir[0], dy = L.dir[1], dz = L.dir[2];
   const double s2 = dx * dx + dy * dy;
   if (!(fabs(dphi) <= 0.02) || !(fabs(dth) <= 0.02) || !(s2 > 1e-12)) {
-    if (absAngles) {
-      stepperUpdate(L, pl, par, cov, mass);
-    } else {
-      double full[6];
-#pragma unroll
-      for (int e = 0; e < 6; ++e) full[e] = par[e];
-      full[2] = atan2(dy, dx) + dphi;
-      full[3] = atan2(sqrt(s2), dz) + dth;
-      stepperUpdate(L, pl, full, cov, mass);
-    }
+    stepperUpdate(L, pl, par, cov, mass);
     return;
   }
 #pragma unroll
@@ -1594,27 +1566,12 @@ static __device__ __forceinline__ bool materialStep(const Params &P, int k, cons
   return kfm::interact(P.planeSlab[k], P.materialEffects, P.planes[k].T, dir, p, q, P.mass, fx);
 }
 
-//
-// Angles of the stored states.  The smoother uses a state's angles only in
-// x_s = x_f + G (x_s' - x_p') (GainMatrixSmoother.hpp:21-94): as the
-// difference of the next state's smoothed and predicted angles, and as this
-// state's filtered angle plus a correction.  So a state after the first may
-// hold its angles as offsets from its own predicted angles (predicted 0,
-// filtered = the gain's correction, smoothed = the smoother's correction):
-// the recursion is unchanged and the first state, which keeps absolute
-// angles, comes out absolute.  The two atan2 of the predicted angles are
-// then evaluated once per track instead of once per surface.  Absolute
-// angles stay where a state's angles are read on their own: smoothed states
-// returned to the caller, the general smoother with material, the adjoint's
-// tape.
 template <typename R, typename H>
 __device__ void filterHit(Lane<R, H> &L, const Params &P, const PlaneD *planes, int k) {
   const PlaneD &pl = planes[k];
   L.hook.hitBegin(L, k);
-  constexpr bool kOffsetForm = std::is_same<H, NoHook>::value;
-  const bool absAngles = !kOffsetForm || L.measStates == 0 || P.oSmoothed != nullptr;
   double pred[6], Jst[25];
-  boundStatePlane(L, pl, pred, Jst, absAngles);
+  boundStatePlane(L, pl, pred, Jst);
   const double *mp = P.meas + (size_t)k * 5 * P.stride + L.idx;
   const double m0 = mp[0], m1 = mp[P.stride], v00 = mp[2 * P.stride],
                v01 = mp[3 * P.stride], v11 = mp[4 * P.stride];
@@ -1688,7 +1645,7 @@ __device__ void filterHit(Lane<R, H> &L, const Params &P, const PlaneD *planes, 
     if (H::kMaterial && P.materialEffects)
       for (int e = 0; e < 21; ++e) *wsCovPtr(P, L, s, 21 + e) = cf[e];
     L.chi2 += chi2;
-    stepperUpdateFiltered(L, pl, pred, filt, cf, P.mass, absAngles);
+    stepperUpdateFiltered(L, pl, pred, filt, cf, P.mass);
     if (!P.faithful) planeJacToGlobal(L, pl);
   }
   if constexpr (H::kMaterial) {

@@ -525,12 +525,12 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
     // of |k| at 2^-24 each and the sums': below 1e-6 |k|) decides unless it
     // comes near the tolerance
     {
-      const float hf = narrow<true>(h);
+      const float hf = narrow(h);
       float e = 0.f;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        const float a = narrow<true>(k1[i]), b = narrow<true>(k2[i]), c = narrow<true>(k3[i]),
-                    d = narrow<true>(k4[i]);
+        const float a = narrow(k1[i]), b = narrow(k2[i]), c = narrow(k3[i]),
+                    d = narrow(k4[i]);
         e += fabsf((a - b) + (d - c)) + 1e-6f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d));
       }
       if (hf * hf * e <= P.tolAcceptF) break;

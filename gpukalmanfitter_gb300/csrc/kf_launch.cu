@@ -133,11 +133,12 @@ struct Spread {
 };
 static Spread spread(int64_t n, int sms) {
   if (n > 0x7f000000) return {32, false, false}; // the queue counts in 32 bits
+  const bool room = n > kSortBuckets + 16;       // for the sort's counts (kf_fit_batch)
   const int64_t full = 32 * (int64_t)sms;
   const int64_t perSm = std::max<int64_t>(kLeastWarps, (n + full - 1) / full);
-  if (perSm > 8) return {32, true, true};
+  if (perSm > 8) return {32, room, room};
   const int lanes = (int)((n + sms * perSm - 1) / (sms * perSm));
-  return {lanes, lanes >= 8, false};
+  return {lanes, room && lanes >= 8, false};
 }
 
 // Batches of up to kCoopMost tracks an SM run eight lanes a track, again as few
@@ -171,7 +172,7 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
     return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
   }
   Spread sp = spread(P.n, sms);
-  if (asked) sp = {32, P.n > kSortBuckets, P.n > kSortBuckets};
+  if (asked) sp = {32, sp.sort || P.n > kSortBuckets + 16, P.n > kSortBuckets + 16};
   P.lanes = sp.lanes;
   if (sp.sort) {
     const int32_t rc = sortQueue(P, q.hist, q.offs, q.perm, q.counter, s);
@@ -183,7 +184,7 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   // with a queue one block of 8 warps an SM (2 % over one-warp blocks: warps
   // that start together share instruction fetches)
   const int block = asked ? shape->bs : sp.queue ? kQueueBlock : kDefaultBlock;
-  P.align = !asked && sp.queue && mixed && !P.materialEffects;
+  P.align = sp.queue && mixed && block == kQueueBlock && !P.materialEffects;
   if (mixed) {
     e = (uniform ? b->mixedUniform : b->mixedGrid)(P, block, s);
   } else if (!uniform) {

@@ -115,13 +115,14 @@ typedef struct kf_config {
                                 form for KF_KERNEL_PERSISTENT and the
                                 thread-per-track grid otherwise; the device-buffer
                                 entry points each run their own form */
-  int32_t block_size;        /* batched form: threads per CTA (64, 128, 256),
-                                0 = 128 */
-  int32_t min_blocks_per_sm; /* batched form: CTAs per SM the persistent kernel
-                                is compiled for (its register budget), 0 = 4;
-                                compiled shapes (threads x CTAs): 128 x 2..5,
-                                64 x 4, 64 x 8, 256 x 1, 256 x 2; kf_autotune
-                                picks one */
+  int32_t block_size;        /* batched form: threads per CTA (64, 128, 256);
+                                with both this and min_blocks_per_sm 0 the
+                                library chooses the launch from the batch's
+                                size; 0 alone = 128 */
+  int32_t min_blocks_per_sm; /* batched form: CTAs per SM the kernel is compiled
+                                for (its register budget), 0 alone = 4; shapes
+                                (threads x CTAs): 128 x 2..5, 64 x 4, 64 x 8,
+                                256 x 1, 256 x 2; kf_autotune picks one */
   int32_t material_effects;  /* bit 0: multiple scattering, bit 1: energy loss
                                 at the surfaces' material (kf_geometry_t.material)
                                 after each filter update (KalmanFitter.hpp:405-449,
