@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kZBlock, 8) adjointZ(const __grid_constant__ P
     if (!L.parked && L.pc != PC_DONE) advance(L, P, sp);
     const bool waiting = L.parked || L.pc == PC_DONE;
     if (__all_sync(0xffffffffu, waiting)) {
-      if (L.parked) runEvent(L, P, sp);
+      if (eventDue(L)) runEvent(L, P, sp);
       if (__all_sync(0xffffffffu, L.pc == PC_DONE)) break;
     }
   }

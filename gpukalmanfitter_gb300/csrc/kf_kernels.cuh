@@ -12,6 +12,7 @@
 // has no hit waits too: passing it would put that lane a plane ahead, and its
 // steps there would run with the others idle (tracks with 10 % holes: 1.24
 // instead of 1.45 times the warp instructions of a track without divergence).
+// Smoothing and the perigee come after the warp's last plane (eventDue).
 //
 // With P.align (the mixed form's queue) the eight warps of a block run each
 // event together: the mixed kernel's code is larger than the instruction
@@ -40,7 +41,7 @@ __device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64
     const bool waiting = L.parked || L.pc == PC_DONE;
     if (__all_sync(0xffffffffu, waiting)) {
       if (align) __syncthreads();
-      if (L.parked) runEvent(L, P, sp);
+      if (eventDue(L)) runEvent(L, P, sp);
       if (align ? __syncthreads_and(L.pc == PC_DONE) : __all_sync(0xffffffffu, L.pc == PC_DONE)) break;
     }
   }
