@@ -91,6 +91,7 @@ struct Params {
   const int32_t *perm;   // queue position -> track index (null: the identity)
   int32_t *queueCounter; // next unclaimed queue position (null: warp w takes the w-th share)
   int lanes;             // tracks per warp
+  int split;             // static shares, or a queue of this many one-warp blocks (kf_kernels.cuh)
   int align;             // with a queue: a block's warps claim tracks and run events together
   // FP64 fit in a uniform field: the field along z of the frame that the
   // planes are given in (rot: its axes, rows; the identity unless rotated)

@@ -3,7 +3,8 @@
 // fitTracks: one thread per track, P.lanes tracks per warp.  With a queue
 // counter a grid of the device's resident capacity whose warps claim their
 // next tracks (sorted longest first) with one atomic until the queue is
-// empty; without, warp w fits the w-th share.  launchFit chooses.
+// empty; without, warp w fits the w-th share.  launchFit chooses, for some
+// sizes the kernel (unevenTracks).
 //
 // Lanes step independently and park at every plane they reach and at other
 // heavy actor work (smoothing, final transport); when every lane of the warp
@@ -58,6 +59,24 @@ __device__ __forceinline__ void fitWarp(const Params &P, const PlaneD *sp, int64
   }
 }
 
+// P.split (batches of 4 ... 8 warps an SM, sorted, one-warp blocks): are the
+// tracks' lengths uneven enough to run one warp on each SM sub-partition,
+// P.split in all, and let these claim the shorter rest as they finish, instead
+// of giving some sub-partitions two warps from the start?  The queue's time is
+// the longest warp's, or that of the shortest first one and what follows it, at
+// a lone warp's 85 cycles per FP64 instruction; two warps that share a
+// sub-partition take 65-70 each.  Measured (FP64 with smoothed states, lengths
+// 5-30: 20011 tracks 1.56 -> 1.49 ms, 30000 1.80 -> 1.51, 38900 (the ratio below
+// at 1.17) 1.99 -> 1.76; mixed, 30000 tracks 1.20 -> 0.98 ms); with one length
+// (the ratio at 2) the queue would lose: uniform field 0.56 -> 0.59 and 0.73 ->
+// 0.78 ms at 20011 and 38900 tracks, material 0.72 -> 0.87 ms at 20011.
+__device__ __forceinline__ bool unevenTracks(const Params &P) {
+  if (!P.nplanes) return false;
+  auto length = [&](int64_t q) { return min(max(P.nplanes[P.perm[q]], 1), P.nSurf); };
+  const int64_t last = 32 * (int64_t)P.split; // the first track past the first warps
+  return last < P.n && 4 * (length(last - 1) + length(last)) <= 5 * length(0);
+}
+
 template <int FORM, bool MAT, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ Params P) {
   // the plane table behind the threads' columns
@@ -65,8 +84,14 @@ __global__ void __launch_bounds__(MAXT, MINB) fitTracks(const __grid_constant__ 
   for (int k = threadIdx.x; k < P.nSurf; k += blockDim.x) sp[k] = P.planes[k];
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const bool queue = P.queueCounter != nullptr, align = P.align != 0;
-  const int lanes = P.lanes;
+  const bool align = P.align != 0;
+  bool queue = P.queueCounter != nullptr;
+  int lanes = P.lanes;
+  if (P.split) {
+    queue = unevenTracks(P);
+    if (queue && blockIdx.x >= P.split) return;
+    if (queue) lanes = 32;
+  }
   __shared__ int claim;
   for (;;) {
     int64_t base;
@@ -125,7 +150,7 @@ template <int FORM> __global__ void __launch_bounds__(32, 8) fitCoop(const __gri
     const int64_t per_block = (int64_t)(bs / 32) * P.lanes;                                  \
     const int64_t need = (P.n + per_block - 1) / per_block;                                  \
     int64_t blocks = need;                                                                   \
-    if (P.queueCounter) {                                                                    \
+    if (P.queueCounter && !P.split) {                                                        \
       int dev = 0, sms = 0, per = 0;                                                         \
       e = cudaGetDevice(&dev);                                                               \
       if (e != cudaSuccess) return e;                                                        \

@@ -117,14 +117,16 @@ static void toFieldFrame(Params &P) {
 }
 
 constexpr int64_t kLeastWarps = 3; // warps an SM that a small batch spreads over
+constexpr int64_t kFillWarps = 4;  // one on each SM sub-partition
 
 // How a batch is laid over the chip.  One FP64 instruction of a warp costs the
 // same whatever its active lanes, each SM sub-partition starts one every 64
 // cycles, and four warps (one a sub-partition) fill an SM's FP64 pipe.  So a
 // batch first spreads over 3 warps on every SM with as few tracks a warp as
 // that takes (fewer lanes to wait for: 1000 map tracks mixed 1530 -> 1393
-// us), then over 4 ... 8 of them, the kernel's residency; beyond that warps
-// of 32 tracks claim work from the queue.  Sorting (3 small kernels, 15 us)
+// us), then over 4 ... 8 of them, the kernel's residency (from 5 on the kernel
+// may take a queue of 4 instead, unevenTracks); beyond that warps of 32
+// tracks claim work from the queue.  Sorting (3 small kernels, 15 us)
 // pays from 8 tracks a warp on.
 struct Spread {
   int lanes;  // tracks per warp
@@ -153,6 +155,7 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   if (!shape) return fail(KF_ERR_UNSUPPORTED, "no fit kernel for this block size / blocks per SM%s");
   cudaError_t e;
   P.lanes = 32;
+  P.split = 0;
   if (P.materialEffects && P.oSmoothed) {
     e = (mixed ? launchFitMaterialStates_mixed : launchFitMaterialStates_fp64)(P, 0, s);
     return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
@@ -179,7 +182,8 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
     if (rc) return rc;
     P.perm = q.perm;
   }
-  if (sp.queue) P.queueCounter = q.counter;
+  if (!sp.queue && sp.sort && P.n > kFillWarps * 32 * sms) P.split = (int)(kFillWarps * sms);
+  if (sp.queue || P.split) P.queueCounter = q.counter;
   const Budget *b = P.materialEffects ? &kMaterial : shape->budget;
   // with a queue one block of 8 warps an SM (2 % over one-warp blocks: warps
   // that start together share instruction fetches)

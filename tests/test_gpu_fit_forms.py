@@ -124,3 +124,20 @@ def test_lanes_per_track_do_not_change_the_bits(kf, n, kind):
     part = kf.fit_device(shard.subset(tel, np.arange(n)), cfg)
     for k, v in part.items():
         assert np.array_equal(v, whole[k][..., :n]), k
+
+
+@pytest.mark.parametrize("n", [19456, 19457, 30011, 38912, 38913])
+@pytest.mark.parametrize("uneven", [False, True])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_shares_or_queue_do_not_change_the_bits(kf, n, uneven, precision):
+    """Batches of 4 ... 8 warps an SM take static shares or, with uneven
+    lengths, a queue of 4 warps an SM; larger ones a queue of 8: the last
+    tracks of the batch come out bitwise as a batch of their own."""
+    kw = dict(n_planes=12, x_first=80., x_step=80., min_len=4 if uneven else 12, max_len=12, hit_prob=0.9)
+    tel = kf.make_telescope(n, seed=36, **kw)
+    from gpukalmanfitter_gb300 import shard
+    cfg = kf.default_config(overstep_limit=0.1, precision=precision)
+    whole = kf.fit_device(tel, cfg)
+    part = kf.fit_device(shard.subset(tel, np.arange(n - 2000, n)), cfg)
+    for k, v in part.items():
+        assert np.array_equal(v, whole[k][..., -2000:]), k
