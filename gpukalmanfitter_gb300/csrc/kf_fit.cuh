@@ -121,7 +121,13 @@ template <> struct LegState<kGrid64> {
 // (applyTransportOffsets)
 template <> struct LegState<kMixed> {};
 template <> struct LegState<kMixedUniform> {};
-template <> struct LegState<kUniform64, 8> : LegState<kUniform64> {};
+// each lane its 2-vector of those that the step turns alike, (v, p) = the
+// track's (dir, pos) in lanes 0 and 1, ((g, -b), (r, -q1)) in 2 and 3, (c, a)
+// in the others
+template <> struct LegState<kUniform64, 8> {
+  double v[2], p[2], s;
+  double y, dx, dy;
+};
 template <> struct LegState<kMixed, 8> {};
 template <> struct LegState<kMixedUniform, 8> {};
 // each lane of a group carries its own column (2: phi, 3: theta, 4: q/p)
@@ -255,7 +261,11 @@ __device__ __forceinline__ void setMomentum(LT &L, const Params &P, double ip, b
 template <int FORM, bool MAT, class H>
 __device__ __forceinline__ void legReset(FitLane<FORM, MAT, H> &L, const Trig &t) {
   L.stepped = false;
-  if constexpr (isUniform(FORM)) {
+  if constexpr (FORM == kUniform64 && H::kGroup > 1) {
+    L.g.v[0] = (threadIdx.x & 6) == 2 ? 1. : 0.;
+    L.g.v[1] = L.g.p[0] = L.g.p[1] = L.g.s = 0.;
+    L.g.y = L.g.dx = L.g.dy = 0.;
+  } else if constexpr (isUniform(FORM)) {
     L.g.g = 1.;
     L.g.b = L.g.r = L.g.q1 = L.g.s = 0.;
     L.g.c[0] = L.g.c[1] = L.g.a[0] = L.g.a[1] = 0.;
@@ -377,31 +387,57 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT, H> &L, const Para
   const double hb = h * P.Bz, hhb = h * hb;
   const double al1 = hb * fma(x, -0.5, 1.), be2 = hb * al;
   const double mu1 = hhb * fma(x, -0.125, 0.5), nu1 = hhb * y * (1. / 3.);
-  // q/p column
-  const double a0 = fma(hn, g.c[0], fma(mu, g.c[1], fma(mu1, dy, fma(-nu1, dx, g.a[0]))));
-  const double a1 = fma(hn, g.c[1], fma(-mu, g.c[0], fma(-mu1, dx, fma(-nu1, dy, g.a[1]))));
-  const double c0 = fma(be1, g.c[0], fma(al, g.c[1], fma(al1, dy, -be2 * dx)));
-  const double c1 = fma(be1, g.c[1], fma(-al, g.c[0], fma(-al1, dx, -be2 * dy)));
-  g.a[0] = a0;
-  g.a[1] = a1;
-  g.c[0] = c0;
-  g.c[1] = c1;
-  // transport of the direction columns
-  g.r = fma(hn, g.g, fma(-mu, g.b, g.r));
-  g.q1 = fma(hn, g.b, fma(mu, g.g, g.q1));
-  g.s += h;
-  const double gg = fma(be1, g.g, -al * g.b);
-  g.b = fma(be1, g.b, al * g.g);
-  g.g = gg;
-  g.y = y;
-  g.dx = dx;
-  g.dy = dy;
-  // the track
-  L.pos[0] = fma(hn, dx, fma(mu, dy, L.pos[0]));
-  L.pos[1] = fma(hn, dy, fma(-mu, dx, L.pos[1]));
-  L.pos[2] = fma(h, L.dir[2], L.pos[2]);
-  L.dir[0] = fma(be1, dx, al * dy);
-  L.dir[1] = fma(be1, dy, -al * dx);
+  if constexpr (H::kGroup > 1) {
+    // this lane's 2-vector (LegState); the q/p column has a source besides (a
+    // product plus -0 rounds as the product)
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    const int l = threadIdx.x & 7;
+    const bool track = l < 2, qp = l >= 4;
+    const double v0 = track ? dx : g.v[0], v1 = track ? dy : g.v[1];
+    const double p0 = track ? L.pos[0] : g.p[0], p1 = track ? L.pos[1] : g.p[1];
+    const double sc0 = fma(al1, dy, -be2 * dx), sc1 = fma(-al1, dx, -be2 * dy);
+    const double sa0 = fma(mu1, dy, fma(-nu1, dx, p0)), sa1 = fma(-mu1, dx, fma(-nu1, dy, p1));
+    g.p[0] = fma(hn, v0, fma(mu, v1, qp ? sa0 : p0));
+    g.p[1] = fma(hn, v1, fma(-mu, v0, qp ? sa1 : p1));
+    g.v[0] = fma(be1, v0, fma(al, v1, qp ? sc0 : -0.));
+    g.v[1] = fma(be1, v1, fma(-al, v0, qp ? sc1 : -0.));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      L.dir[i] = __shfl_sync(group, g.v[i], 0, 8);
+      L.pos[i] = __shfl_sync(group, g.p[i], 0, 8);
+    }
+    L.pos[2] = fma(h, L.dir[2], L.pos[2]);
+    g.s += h;
+    g.y = y;
+    g.dx = dx;
+    g.dy = dy;
+  } else {
+    // q/p column
+    const double a0 = fma(hn, g.c[0], fma(mu, g.c[1], fma(mu1, dy, fma(-nu1, dx, g.a[0]))));
+    const double a1 = fma(hn, g.c[1], fma(-mu, g.c[0], fma(-mu1, dx, fma(-nu1, dy, g.a[1]))));
+    const double c0 = fma(be1, g.c[0], fma(al, g.c[1], fma(al1, dy, -be2 * dx)));
+    const double c1 = fma(be1, g.c[1], fma(-al, g.c[0], fma(-al1, dx, -be2 * dy)));
+    g.a[0] = a0;
+    g.a[1] = a1;
+    g.c[0] = c0;
+    g.c[1] = c1;
+    // transport of the direction columns
+    g.r = fma(hn, g.g, fma(-mu, g.b, g.r));
+    g.q1 = fma(hn, g.b, fma(mu, g.g, g.q1));
+    g.s += h;
+    const double gg = fma(be1, g.g, -al * g.b);
+    g.b = fma(be1, g.b, al * g.g);
+    g.g = gg;
+    g.y = y;
+    g.dx = dx;
+    g.dy = dy;
+    // the track
+    L.pos[0] = fma(hn, dx, fma(mu, dy, L.pos[0]));
+    L.pos[1] = fma(hn, dy, fma(-mu, dx, L.pos[1]));
+    L.pos[2] = fma(h, L.dir[2], L.pos[2]);
+    L.dir[0] = fma(be1, dx, al * dy);
+    L.dir[1] = fma(be1, dy, -al * dx);
+  }
   if (!(akey(x) < 0x3ee4f8b588e368f1LL)) { // |x| >= 1e-5
     const double f = unitFactor(L.dir);
     L.dir[0] *= f;
@@ -783,7 +819,25 @@ __device__ __forceinline__ typename std::enable_if<isUniform(FORM)>::type
 legColumn(const FitLane<FORM, MAT, H> &L, const Params &P, const Trig &t, double o, int c, double p[3],
           double v[3]) {
   using LT = FitLane<FORM, MAT, H>;
-  const auto &g = L.g;
+  LegState<kUniform64> g;
+  if constexpr (H::kGroup > 1) { // from the lanes that carry them (the whole group calls)
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    double m[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      m[i] = __shfl_sync(group, L.g.v[i], c, 8);
+      m[2 + i] = __shfl_sync(group, L.g.p[i], c, 8);
+    }
+    g.g = g.c[0] = m[0];
+    g.c[1] = m[1];
+    g.b = -m[1];
+    g.r = g.a[0] = m[2];
+    g.a[1] = m[3];
+    g.q1 = -m[3];
+    g.s = L.g.s;
+  } else {
+    g = L.g;
+  }
   if (c == 4) {
     p[0] = g.a[0];
     p[1] = g.a[1];
@@ -1168,13 +1222,26 @@ __device__ __forceinline__ void updateState(LT &L, const Params &P, const PlaneD
       sn = fma(d * d2, fma(d2, fma(d2, -1. / 5040., 1. / 120.), -1. / 6.), d);
       cs = fma(d2, fma(d2, fma(d2, fma(d2, 1. / 40320., -1. / 720.), 1. / 24.), -0.5), 1.);
     };
-    double sdp, cdp, sdt, cdt;
-    sinCosSmall(dphi, sdp, cdp);
-    sinCosSmall(dth, sdt, cdt);
-    cP = t.cP * cdp - t.sP * sdp;
-    sP = t.sP * cdp + t.cP * sdp;
-    sT = t.sT * cdt + t.cT * sdt;
-    cT = t.cT * cdt - t.sT * sdt;
+    if constexpr (LT::kCoop) { // phi in the even lanes, theta in the odd ones
+      const unsigned group = 0xffu << (threadIdx.x & 24);
+      const bool odd = threadIdx.x & 1;
+      const double c0 = odd ? t.cT : t.cP, s0 = odd ? t.sT : t.sP;
+      double sd, cd;
+      sinCosSmall(odd ? dth : dphi, sd, cd);
+      const double cn = c0 * cd - s0 * sd, sn = s0 * cd + c0 * sd;
+      cP = __shfl_sync(group, cn, 0, 8);
+      sP = __shfl_sync(group, sn, 0, 8);
+      cT = __shfl_sync(group, cn, 1, 8);
+      sT = __shfl_sync(group, sn, 1, 8);
+    } else {
+      double sdp, cdp, sdt, cdt;
+      sinCosSmall(dphi, sdp, cdp);
+      sinCosSmall(dth, sdt, cdt);
+      cP = t.cP * cdp - t.sP * sdp;
+      sP = t.sP * cdp + t.cP * sdp;
+      sT = t.sT * cdt + t.cT * sdt;
+      cT = t.cT * cdt - t.sT * sdt;
+    }
   }
   const double d[3] = {cP * sT, sP * sT, cT};
   toFrame<LT>(P, d, L.dir);

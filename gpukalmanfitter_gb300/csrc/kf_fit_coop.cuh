@@ -7,12 +7,16 @@
 // group run the same track, each with the whole state; what a hit does per
 // column of the five bound parameters is shared out: lane c forms column c of
 // the bound Jacobian and of F <- J F, entry c of C h and row c of the
-// covariance update, and in a field map transports column c through the RK
-// stages.  About 240 instead of 430 FP64 instructions a hit, and in a field map
-// 340 instead of 450 a step.  Every sum keeps its order, so that the results
-// have the bits of the one-lane form (kf_fit.cuh), which serves larger
-// batches: four tracks a warp are the better use of a warp only while warps
-// are short (launchFit).
+// covariance update; the three sums of h C h^T, and the two angles' updates,
+// go to one lane each.  In a field map lane c transports column c through the
+// RK stages; in a uniform field the track, the leg's scalars and its q/p
+// column, which a step turns alike, are a lane's each.  About 200 instead of
+// 430 FP64 instructions a hit, in a field map 340 instead of 450 a step, in a
+// uniform field 55 instead of 70 (the last two and the sums: 5 tracks of 10
+// planes 205 -> 189 us, 1000 tracks 339 -> 310 us).  Every sum keeps its
+// order, so that the results have the bits of the one-lane form (kf_fit.cuh),
+// which serves larger batches: four tracks a warp are the better use of a warp
+// only while warps are short (launchFit).
 //
 // The lanes of a group take every branch together; shared-memory exchange is
 // separated by __syncwarp of the group.
@@ -73,17 +77,17 @@ __device__ __forceinline__ void boundColumn(const CoopLane<FORM> &L, const Param
       const bool th = c == 3;
       const double e0 = th ? tl.cT * tl.cP : -tl.sT * tl.sP, e1 = th ? tl.cT * tl.sP : tl.sT * tl.cP,
                    e2 = th ? -tl.sT : 0.;
-      p[0] = fma(g.r, e0, g.q1 * e1);
-      p[1] = fma(g.r, e1, -g.q1 * e0);
+      p[0] = fma(g.p[0], e0, -g.p[1] * e1);
+      p[1] = fma(g.p[0], e1, g.p[1] * e0);
       p[2] = g.s * e2;
-      v[0] = fma(g.g, e0, g.b * e1);
-      v[1] = fma(g.g, e1, -g.b * e0);
+      v[0] = fma(g.v[0], e0, -g.v[1] * e1);
+      v[1] = fma(g.v[0], e1, g.v[1] * e0);
       v[2] = e2;
       if (c == 4) {
-        p[0] = g.a[0];
-        p[1] = g.a[1];
-        v[0] = g.c[0];
-        v[1] = g.c[1];
+        p[0] = g.p[0];
+        p[1] = g.p[1];
+        v[0] = g.v[0];
+        v[1] = g.v[1];
         p[2] = v[2] = 0.;
       }
       if (first && c == 2) {
@@ -189,7 +193,7 @@ __device__ __forceinline__ void filterHit(CoopLane<FORM> &L, const Params &P, co
   }
   __syncwarp(group);
   // w = C h: this lane's entry
-  double h0[5], h1[5], w0[5], w1[5], Cr[5];
+  double h0[5], h1[5], w0[5], w1[5], wc[2], Cr[5];
 #pragma unroll
   for (int l = 0; l < 5; ++l) {
     h0[l] = L.F(0, l);
@@ -203,8 +207,8 @@ __device__ __forceinline__ void filterHit(CoopLane<FORM> &L, const Params &P, co
       a = fma(Cr[j], h0[j], a);
       b = fma(Cr[j], h1[j], b);
     }
-    L.cold(kCoopScratch) = a;
-    L.cold(kCoopScratch + 1) = b;
+    L.cold(kCoopScratch) = wc[0] = a;
+    L.cold(kCoopScratch + 1) = wc[1] = b;
   }
   __syncwarp(group);
 #pragma unroll
@@ -212,23 +216,27 @@ __device__ __forceinline__ void filterHit(CoopLane<FORM> &L, const Params &P, co
     w0[l] = L.coldOf(kCoopScratch, l);
     w1[l] = L.coldOf(kCoopScratch + 1, l);
   }
-  double a00 = h0[0] * w0[0], a01 = h1[0] * w0[0], a11 = h1[0] * w1[0];
+  // h0 . w0, h1 . w0, h1 . w1: lanes 0, 1, 2 (the others as lane 2)
+  const int l8 = threadIdx.x & 7;
+  double a00, a01, a11;
+  {
+    double hw = (l8 == 0 ? h0[0] : h1[0]) * (l8 < 2 ? w0[0] : w1[0]);
 #pragma unroll
-  for (int i = 1; i < 5; ++i) {
-    a00 = fma(h0[i], w0[i], a00);
-    a01 = fma(h1[i], w0[i], a01);
-    a11 = fma(h1[i], w1[i], a11);
+    for (int i = 1; i < 5; ++i)
+      hw = fma(l8 == 0 ? h0[i] : h1[i], l8 < 2 ? w0[i] : w1[i], hw);
+    a00 = __shfl_sync(group, hw, 0, 8);
+    a01 = __shfl_sync(group, hw, 1, 8);
+    a11 = __shfl_sync(group, hw, 2, 8);
   }
   const Gain g = gain(a00 + v00, a01 + v01, a11 + v11, m0 - x0, m1 - x1);
   const bool outlier = isOutlier(P, g.chi2);
   Trig tn = tr;
   if (!outlier) {
-    double dl[5], dlc = 0., w0c = 0., w1c = 0.;
+    // this lane's entries
+    const double w0c = wc[0], w1c = fma(-g.l, w0c, wc[1]), dlc = fma(w0c, g.e0, wc[1] * g.e1);
+    double dl[5];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      dl[i] = fma(w0[i], g.e0, w1[i] * g.e1);
-      dlc = c == i ? dl[i] : dlc;
-    }
+    for (int i = 0; i < 5; ++i) dl[i] = __shfl_sync(group, dlc, i, 8);
     double w50 = 0., w51 = 0.;
     if (L.timeCorr) {
 #pragma unroll
@@ -237,18 +245,14 @@ __device__ __forceinline__ void filterHit(CoopLane<FORM> &L, const Params &P, co
         w51 = fma(L.Ct(j), h1[j], w51);
       }
     }
-    double dphi = L.F(2, 0) * dl[0], dth = L.F(3, 0) * dl[0];
+    // phi in the even lanes, theta in the odd ones
+    const int r = 2 + (l8 & 1);
+    double da = L.F(r, 0) * dl[0];
 #pragma unroll
-    for (int l = 1; l < 5; ++l) {
-      dphi = fma(L.F(2, l), dl[l], dphi);
-      dth = fma(L.F(3, l), dl[l], dth);
-    }
+    for (int l = 1; l < 5; ++l) da = fma(L.F(r, l), dl[l], da);
+    const double dphi = __shfl_sync(group, da, 0, 8), dth = __shfl_sync(group, da, 1, 8);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      w1[i] = fma(-g.l, w0[i], w1[i]);
-      w0c = c == i ? w0[i] : w0c;
-      w1c = c == i ? w1[i] : w1c;
-    }
+    for (int i = 0; i < 5; ++i) w1[i] = __shfl_sync(group, w1c, i, 8);
     const double a0 = w0c * g.i0, a1 = w1c * g.i1;
     if (own) {
       L.D(c) += dlc;

@@ -144,9 +144,9 @@ static Spread spread(int64_t n, int sms) {
 }
 
 // Batches of up to kCoopMost tracks an SM run eight lanes a track, again as few
-// tracks a warp as kLeastWarps warps an SM allow (the line is where five such
-// warps of four tracks an SM cost as much as 3 warps of 7 lanes: 3000 tracks of
-// 10 planes 418 against 458 us, 3600 tracks 503 against 485 us).
+// tracks a warp as kLeastWarps warps an SM allow (the line is at five such
+// warps of four tracks an SM: 3040 tracks of 10 planes 361 us, 3041 one lane a
+// track 449 us; in the field map 1.86 and 2.25 ms, mixed 1.08 and 1.23 ms).
 constexpr int64_t kCoopMost = 20;
 
 int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers &q, cudaStream_t s) {
