@@ -4,7 +4,9 @@
 //
 // Objective: chi2 = sum over tracks and non-outlier measurement states of
 // (m - H x_s)^T V^-1 (m - H x_s), x_s the smoothed parameters of the fit
-// (closed-form RTS smoother).  One thread per track, tracks in work-queue
+// (closed-form RTS smoother).  With the field along z kf_adjoint_z.cu's kernel
+// serves the call, and the kernel here the tracks whose tape runs over there
+// and other field directions.  One thread per track, tracks in work-queue
 // order (sorted by sequence length and curvature, kfh::sortQueue, so that a
 // warp's lanes take similar numbers of RK steps between surfaces); the
 // adjoint's own workspace is indexed by queue position (coalesced), inputs,

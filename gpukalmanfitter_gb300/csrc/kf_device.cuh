@@ -1,5 +1,11 @@
 // kf_device.cuh — per-track fitter state machine for sm_103a.
 //
+// The navigation, step constraints, field lookups and the propagation loop
+// here serve every kernel; Lane<R>, which transports the covariance from plane
+// to plane, serves the fits with material whose smoothed states are returned
+// (kf_fit_material_states.cu) and the general adjoint (kf_adjoint.cu).  The
+// other fits run kf_fit.cuh's lane.
+//
 // One thread owns one track.  The arithmetic restates the reference
 // KalmanFitter hot path (paths relative to the reference project root):
 //   EigenStepper::step              Propagator/EigenStepper.ipp:226-332

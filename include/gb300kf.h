@@ -88,7 +88,7 @@ enum kf_field_kind {
 enum kf_kernel_kind {
   KF_KERNEL_AUTO = 0,
   KF_KERNEL_THREAD_PER_TRACK = 1, /* one thread per track, grid over tracks */
-  KF_KERNEL_PERSISTENT = 2        /* persistent CTAs pulling a sorted queue */
+  KF_KERNEL_PERSISTENT = 2        /* resident CTAs pulling a sorted queue */
 };
 
 /* Steering of the fit: PropagatorOptions (Propagator.hpp:52-111) plus
@@ -263,8 +263,9 @@ int32_t kf_fit_batch_host(const kf_inputs_t *host_in, kf_outputs_t *host_out,
  * (Run/GPU/Kernels.cu:6-45 from Run/GPU/KalmanFitterGPUTest.cu:461-472) for
  * large batches with uneven track lengths, holes and outliers: tracks are
  * ordered by expected work (sequence length, then |q/p|; longest first) by a
- * counting sort on the device, and a persistent kernel (one resident grid,
- * warps claiming 32 queue positions at a time) fits them.  Results are the
+ * counting sort on the device, and one resident grid, whose warps claim 32
+ * queue positions at a time, fits them (batches too small to fill the device
+ * are spread over it instead, as kf_fit_batch spreads them).  Results are the
  * same as kf_fit_batch's; the workspace is kf_batch_workspace_size bytes. */
 size_t kf_batch_workspace_size(const kf_config_t *cfg, int64_t n_tracks,
                                int32_t n_surfaces);
@@ -273,8 +274,7 @@ int32_t kf_fit_batch_sorted(const kf_inputs_t *in, kf_outputs_t *out,
                             const kf_field_t *field, void *workspace,
                             size_t workspace_bytes, void *stream);
 
-/* A plan captures the whole batched pipeline (queue reset, sort, persistent
- * fit) for fixed buffers into a CUDA graph; each launch replays it with one
+/* A plan captures the whole batched pipeline (queue reset, sort, fit) for fixed buffers into a CUDA graph; each launch replays it with one
  * call.  `stream` must be a created stream (capture is not possible on the
  * legacy default stream).  The buffers must outlive the plan. */
 typedef struct kf_batch_plan kf_batch_plan_t;
@@ -286,7 +286,7 @@ int32_t kf_batch_plan_create(kf_batch_plan_t **plan, const kf_inputs_t *in,
 int32_t kf_batch_plan_launch(kf_batch_plan_t *plan, void *stream);
 void kf_batch_plan_destroy(kf_batch_plan_t *plan);
 
-/* Times every compiled persistent-kernel shape (threads per CTA and CTAs per
+/* Times every compiled kernel shape (threads per CTA and CTAs per
  * SM, see kf_config_t.min_blocks_per_sm) of cfg->precision on the first min(n, 524288) tracks of the batch
  * (best of three runs after a warm-up) and returns the fastest configuration
  * in *tuned (and its time per fit of the sample in *best_ms).  Overwrites
