@@ -22,7 +22,7 @@
 // stores and differentiates J C J^T per plane and whose step records carry the
 // transport Jacobian as 25 words) a plane costs a third of the FP64
 // instructions and a quarter of the tape: 65536 tracks of 20 planes, call and
-// results on the host, 16.2 -> 6.4 ms.
+// results on the host, 16.1 -> 6.3 ms.
 
 #include <cuda_runtime.h>
 
