@@ -130,7 +130,8 @@ template <> struct LegState<kUniform64, 8> {
 };
 template <> struct LegState<kMixed, 8> {};
 template <> struct LegState<kMixedUniform, 8> {};
-// each lane of a group carries its own column (2: phi, 3: theta, 4: q/p)
+// each lane of a group carries its own column (2: phi, 3: theta, 4: q/p, 5: the
+// direction that the leg started with, see legRebase)
 template <> struct LegState<kGrid64, 8> {
   double p[3], v[3], s, k4[3];
 };
@@ -272,11 +273,11 @@ __device__ __forceinline__ void legReset(FitLane<FORM, MAT, H> &L, const Trig &t
     L.g.y = L.g.dx = L.g.dy = 0.;
   } else if constexpr (FORM == kGrid64 && H::kGroup > 1) {
     const int c = threadIdx.x & 7;
-    const bool phi = c == 2, th = c == 3;
+    const bool phi = c == 2, th = c == 3, rad = c == 5;
     L.g.p[0] = L.g.p[1] = L.g.p[2] = 0.;
-    L.g.v[0] = phi ? -t.sT * t.sP : (th ? t.cT * t.cP : 0.);
-    L.g.v[1] = phi ? t.sT * t.cP : (th ? t.cT * t.sP : 0.);
-    L.g.v[2] = th ? -t.sT : 0.;
+    L.g.v[0] = phi ? -t.sT * t.sP : (th ? t.cT * t.cP : (rad ? t.sT * t.cP : 0.));
+    L.g.v[1] = phi ? t.sT * t.cP : (th ? t.cT * t.sP : (rad ? t.sT * t.sP : 0.));
+    L.g.v[2] = th ? -t.sT : (rad ? t.cT : 0.);
     L.g.s = 0.;
     L.g.k4[0] = L.g.k4[1] = L.g.k4[2] = 0.;
   } else if constexpr (FORM == kGrid64) {
@@ -301,6 +302,72 @@ __device__ __forceinline__ void legReset(FitLane<FORM, MAT, H> &L, const Trig &t
     L.Jb = 0.f;
     L.sTr = 0.;
   }
+}
+
+// Field map, faithful_jacobian = 0: where the track runs out of planes, the
+// smoothed state's jacToGlobal takes the place of the last hit's under a leg
+// that has begun (finalizeSmooth).  The leg's transport of any direction is
+// that of the last hit's phi and theta columns and of the leg's first
+// direction itself; the last is carried only in such a fit, in the record of
+// the state that the leg may still reach (a group's lane 5 has it for nothing).
+template <class LT> __device__ __forceinline__ bool keepsDirection(const LT &L, const Params &P) {
+  return !P.faithful && P.smoothing && !L.smoothed && L.measStates > 0 && L.measStates < P.nSurf;
+}
+// the columns phi and theta at `t` in place of those at `t0`
+template <bool MAT, class H>
+__device__ __forceinline__ void legRebase(FitLane<kGrid64, MAT, H> &L, const Params &P, const Trig &t0,
+                                          const Trig &t) {
+  const double is2 = 1. / (t0.sT * t0.sT);
+  const double d0[3] = {t0.sT * t0.cP, t0.sT * t0.sP, t0.cT};
+  const double ph0[3] = {-t0.sT * t0.sP, t0.sT * t0.cP, 0.}, th0[3] = {t0.cT * t0.cP, t0.cT * t0.sP, -t0.sT};
+  double np[2][3], nv[2][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double p[3], v[3]; // of ph0, th0, d0
+    if constexpr (H::kGroup > 1) {
+      const unsigned group = 0xffu << (threadIdx.x & 24);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        p[k] = __shfl_sync(group, L.g.p[i], k < 2 ? 2 + k : 5, 8);
+        v[k] = __shfl_sync(group, L.g.v[i], k < 2 ? 2 + k : 5, 8);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        p[k] = L.g.p[k][i];
+        v[k] = L.g.v[k][i];
+      }
+      p[2] = *recPtr(P, L, L.measStates, i);
+      v[2] = *recPtr(P, L, L.measStates, 3 + i);
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const double e[3] = {c ? t.cT * t.cP : -t.sT * t.sP, c ? t.cT * t.sP : t.sT * t.cP, c ? -t.sT : 0.};
+      double a[3] = {0., 0., 0.};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        a[0] += e[k] * ph0[k] * is2;
+        a[1] += e[k] * th0[k];
+        a[2] += e[k] * d0[k];
+      }
+      np[c][i] = a[0] * p[0] + a[1] * p[1] + a[2] * p[2];
+      nv[c][i] = a[0] * v[0] + a[1] * v[1] + a[2] * v[2];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if constexpr (H::kGroup > 1) {
+        if ((threadIdx.x & 7) == 2 + c) {
+          L.g.p[i] = np[c][i];
+          L.g.v[i] = nv[c][i];
+        }
+      } else {
+        L.g.p[c][i] = np[c][i];
+        L.g.v[c][i] = nv[c][i];
+      }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -621,6 +688,20 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
     column(g.p[0], g.v[0], false, 0.);
     column(g.p[1], g.v[1], false, 0.);
     column(g.p[2], g.v[2], true, iq);
+    if (keepsDirection(L, P)) {
+      double p[3], v[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        p[i] = L.stepped ? *recPtr(P, L, L.measStates, i) : 0.;
+        v[i] = L.stepped ? *recPtr(P, L, L.measStates, 3 + i) : L.dir[i];
+      }
+      column(p, v, false, 0.);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        *recPtr(P, L, L.measStates, i) = p[i];
+        *recPtr(P, L, L.measStates, 3 + i) = v[i];
+      }
+    }
   }
   g.s += h;
 #pragma unroll
@@ -1680,9 +1761,13 @@ __device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT, H> &L, const P
   updateState(L, P, pl, x[0], x[1], t, x[2], x[3], qop, true);
   if (!P.faithful) {
     // jacToGlobal from the smoothed state's own plane and direction
+    const Trig t0 = trigLoad(L);
     trigSave(L, t);
     L.lastPlane = L.firstPlane;
-    if (FORM == kGrid64) legReset(L, t);
+    if constexpr (FORM == kGrid64) {
+      if (L.stepped) legRebase(L, P, t0, t);
+      else legReset(L, t);
+    }
   }
   // (a leg that had begun when the track ran out of planes goes on)
   L.t = fma(-legPath(L), L.dtds, tm);

@@ -1,0 +1,58 @@
+"""Calls at the edges of what the entry points take: tracks that run out of
+planes, values that are not finite, option fields that a form ignores.  The
+oracle, or the same call in another form, says what each has to give."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+DIAG = [0, 6, 11, 15, 18, 20]
+PAIRS = [(i, j) for i in range(6) for j in range(i, 6)]
+
+
+def _cov_deviation(g, o, sel):
+    """Largest covariance deviation in units of sigma_i sigma_j."""
+    sig = np.sqrt(np.abs(o["cov"][DIAG][:, sel]))
+    return max(np.max(np.abs(g["cov"][e] - o["cov"][e])[sel] / (sig[i] * sig[j]), initial=0.)
+               for e, (i, j) in enumerate(PAIRS))
+
+
+def _in_constant_map(tel, kf):
+    """The telescope with its uniform field as a map of equal values; the
+    field is first rounded to the map's FP32."""
+    import copy
+    bz = np.float32(tel.bz_tesla * kf.TESLA)
+    tel.bz_tesla = float(bz) / kf.TESLA
+    m = copy.copy(tel)
+    grid = np.zeros((8, 4), np.float32)
+    grid[:, 2] = bz
+    m.field_grid, m.field_n, m.field_half = grid.reshape(-1), 2, 2000.
+    return m
+
+
+# Tracks that miss their last planes (with a short overstep limit the stepper
+# passes some) end the forward fit between planes; their results are written,
+# with the status of the missing measurement.  A map of one value is the
+# uniform field, whose kernels form the leg's transport in another way; the
+# bound is the 1e-9 of the parity tests.
+@pytest.mark.parametrize("n", [2000, 4000])  # eight lanes a track, one lane a track
+@pytest.mark.parametrize("faithful", [0, 1])
+@pytest.mark.parametrize("material, smoothed", [(0., False), (0., True), (0.3, False)])
+def test_tracks_that_miss_their_last_planes(kf, n, faithful, material, smoothed):
+    tel = kf.make_telescope(n, seed=81, n_planes=15, x_first=80., x_step=80., min_len=5, max_len=15,
+                            hit_prob=0.9)
+    tel.material = np.tile(kf.silicon(material), (15, 1)) if material else None
+    cfg = kf.default_config(overstep_limit=0.01, faithful_jacobian=faithful,
+                            material_effects=3 if material else 0)
+    m = _in_constant_map(tel, kf)
+    o = kf.fit_device(tel, cfg, smoothed=smoothed)
+    g = kf.fit_device(m, cfg, smoothed=smoothed)
+    for k in ("status", "n_meas", "n_steps"):
+        assert np.array_equal(g[k], o[k]), k
+    written = (o["cov"][0] != 0.) & (o["status"] != 0)
+    assert written.sum() > 20
+    sig = np.sqrt(np.abs(o["cov"][DIAG][:, written]))
+    dev = np.abs(g["params"] - o["params"])[:, written] / np.maximum(np.abs(o["params"][:, written]), sig)
+    print(written.sum(), dev.max(), _cov_deviation(g, o, written))
+    assert dev.max() < 1e-9
+    assert _cov_deviation(g, o, written) < 1e-9
