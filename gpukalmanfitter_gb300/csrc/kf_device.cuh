@@ -125,11 +125,18 @@ __device__ __forceinline__ void cross3(const T a[3], const T b[3], T r[3]) {
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 
-// an FP32 value as FP64 on the integer pipe (normal values exactly; FP32
-// zeros and denormals come out below 1.2e-38)
-__device__ __forceinline__ double widen(float f) {
+// an FP32 value as FP64 on the integer pipe: normal values exactly, FP32 zeros
+// and denormals below 1.2e-38; widenFinite: infinities and NaN come out finite
+__device__ __forceinline__ double widenFinite(float f) {
   const int b = __float_as_int(f);
   return __hiloint2double(((b >> 3) & 0x8fffffff) + 0x38000000, b << 29);
+}
+// infinities and NaN too
+__device__ __forceinline__ double widen(float f) {
+  const int b = __float_as_int(f);
+  int hi = ((b >> 3) & 0x8fffffff) + 0x38000000;
+  if ((b & 0x7f800000) == 0x7f800000) hi |= 0x7ff00000;
+  return __hiloint2double(hi, b << 29);
 }
 
 // FP64 to FP32, rounded to nearest even, on the integer pipe (a conversion
@@ -679,7 +686,8 @@ __device__ __forceinline__ void rkFirstDelta(const FieldD &F, const float posf[3
   double B[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    B[i] = widen(S.Bf[i].hi) + widen(S.Bf[i].lo);
+    // (a value that is not finite rejects the step by the error estimates)
+    B[i] = widenFinite(S.Bf[i].hi) + widenFinite(S.Bf[i].lo);
     S.s.Bf[i] = S.Bf[i].hi;
   }
   double c[3];

@@ -565,26 +565,27 @@ __device__ __forceinline__ void fieldScaled(const FieldD &F, const double p[3], 
   // The differences of neighbours along x are taken in FP32, where they are
   // exact for values within a factor of 2 of each other (Sterbenz), as almost
   // all are; TwoSum's error term tells, and any inexact one sends the lookup
-  // through FP64 differences: 12 of 42 FP64 instructions a lookup less.
-  float off = 0.f;
+  // through FP64 differences: 12 of 42 FP64 instructions a lookup less.  A
+  // value or difference that is not finite makes the term NaN.
+  unsigned off = 0;
   auto dif = [&](float a, float b) {
     const float e = __fsub_rn(b, a), t = __fsub_rn(e, b);
-    off = fmaxf(off, fabsf(__fsub_rn(__fsub_rn(b, __fsub_rn(e, t)), __fadd_rn(a, t))));
-    return widen(e);
+    off |= __float_as_uint(__fsub_rn(__fsub_rn(b, __fsub_rn(e, t)), __fadd_rn(a, t)));
+    return widenFinite(e);
   };
   auto mix = [](double a, double b, double w) { return fma(w, b - a, a); };
   auto tri = [&](float a000, float a100, float a010, float a110, float a001, float a101,
                  float a011, float a111) {
-    const double c00 = fma(f[0], dif(a000, a100), widen(a000));
-    const double c10 = fma(f[0], dif(a010, a110), widen(a010));
-    const double c01 = fma(f[0], dif(a001, a101), widen(a001));
-    const double c11 = fma(f[0], dif(a011, a111), widen(a011));
+    const double c00 = fma(f[0], dif(a000, a100), widenFinite(a000));
+    const double c10 = fma(f[0], dif(a010, a110), widenFinite(a010));
+    const double c01 = fma(f[0], dif(a001, a101), widenFinite(a001));
+    const double c11 = fma(f[0], dif(a011, a111), widenFinite(a011));
     return mix(mix(c00, c10, f[1]), mix(c01, c11, f[1]), f[2]) * s;
   };
   B[0] = tri(v000.x, v100.x, v010.x, v110.x, v001.x, v101.x, v011.x, v111.x);
   B[1] = tri(v000.y, v100.y, v010.y, v110.y, v001.y, v101.y, v011.y, v111.y);
   B[2] = tri(v000.z, v100.z, v010.z, v110.z, v001.z, v101.z, v011.z, v111.z);
-  if (!(off == 0.f)) {
+  if (off & 0x7fffffffu) { // (a zero's sign apart)
     auto tri64 = [&](float a000, float a100, float a010, float a110, float a001, float a101,
                      float a011, float a111) {
       const double c00 = mix(widen(a000), widen(a100), f[0]), c10 = mix(widen(a010), widen(a110), f[0]);
@@ -794,13 +795,14 @@ rkStep(FitLane<FORM, MAT, H> &L, const Params &P) {
   L.sTr += h;
   // motion: FP64 state, FP64 k1, FP32 sums of the offsets
   //   pos += h d + h^2/6 (3 k1 + d2 + d3),  dir += h/6 (6 k1 + 2 (d2 + d3) + d4)
+  // (finite: any other offset makes either error estimate NaN or infinite)
   const double h6 = h * (1. / 6.), hh6 = h * h6;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float s23 = S.d2[i] + S.d3[i];
     const float s234 = 2.f * s23 + S.d4[i];
-    L.pos[i] = fma(hh6, fma(3., S.k1[i], widen(s23)), fma(h, L.dir[i], L.pos[i]));
-    L.dir[i] = fma(h6, fma(6., S.k1[i], widen(s234)), L.dir[i]);
+    L.pos[i] = fma(hh6, fma(3., S.k1[i], widenFinite(s23)), fma(h, L.dir[i], L.pos[i]));
+    L.dir[i] = fma(h6, fma(6., S.k1[i], widenFinite(s234)), L.dir[i]);
   }
   const double f = unitFactor(L.dir);
   L.dir[0] *= f;
@@ -1208,6 +1210,7 @@ boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
     for (int c = 0; c < 5; ++c) R3[c] = (c == 4 ? L.Jb : 0.f);
   }
   const float *U = pl.Uf, *V = pl.Vf;
+  float bad = 0.f; // NaN where an entry is not finite
   const float f24 = narrow(j24), f25 = narrow(j25), f34 = narrow(j34), f35 = narrow(j35), f36 = narrow(j36);
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
@@ -1215,7 +1218,8 @@ boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
     const float e1 = V[0] * dP[0][c] + V[1] * dP[1][c] + V[2] * dP[2][c];
     const float e2 = f24 * dD[0][c] + f25 * dD[1][c];
     const float e3 = f34 * dD[0][c] + f35 * dD[1][c] + f36 * dD[2][c];
-    const double w0 = widen(e0), w1 = widen(e1), w2 = widen(e2), w3 = widen(e3);
+    bad = fmaf(e0, 0.f, fmaf(e1, 0.f, fmaf(e2, 0.f, fmaf(e3, 0.f, bad))));
+    const double w0 = widenFinite(e0), w1 = widenFinite(e1), w2 = widenFinite(e2), w3 = widenFinite(e3);
     if (c >= 2) { // (a shift on the last plane has no field-induced part)
       J[0][c] = c < 4 ? J[0][c] + w0 : w0;
       J[1][c] = c < 4 ? J[1][c] + w1 : w1;
@@ -1224,6 +1228,7 @@ boundJacobian(const FitLane<FORM, MAT, H> &L, const Params &P,
     J[3][c] = c >= 2 && c < 4 ? J[3][c] + w3 : w3;
     if (time) J5[c] = (double)R3[c];
   }
+  if (bad != 0.f) J[0][0] = __longlong_as_double(0x7ff8000000000000LL); // and with it the gain
 }
 
 // ---------------------------------------------------------------------------
@@ -1368,7 +1373,9 @@ __device__ __forceinline__ double crossMaterial(const kfm::Slab &sl, int flags, 
 
 // any of a Jacobian's entries infinite or NaN (the smoother's NaN gain), on
 // the integer pipe
-__device__ __forceinline__ bool anyBad(const double (&J)[4][5]) {
+template <int FORM> __device__ __forceinline__ bool anyBad(const double (&J)[4][5]) {
+  // (boundJacobian's own check of the mixed form's)
+  if (isMixed(FORM)) return ((unsigned)__double2hiint(J[0][0]) & 0x7fffffffu) >= 0x7ff00000u;
   unsigned m = 0;
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -1417,7 +1424,7 @@ __device__ __forceinline__ void filterHit(FitLane<FORM, MAT, H> &L, const Params
   double J[4][5], J5[5] = {0., 0., 0., 0., 0.};
   Trig tr;
   boundJacobian(L, P, planes, pl, time, tr, J, J5);
-  if (!first && anyBad(J)) L.badJ = true;
+  if (!first && anyBad<FORM>(J)) L.badJ = true;
   if (time) L.t = fma(legPath(L), L.dtds, L.t);
   const double d0 = L.pos[0] - pl.c[0], d1 = L.pos[1] - pl.c[1], d2 = L.pos[2] - pl.c[2];
   const double x0 = pl.U[0] * d0 + pl.U[1] * d1 + pl.U[2] * d2;

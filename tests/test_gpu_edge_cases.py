@@ -56,3 +56,21 @@ def test_tracks_that_miss_their_last_planes(kf, n, faithful, material, smoothed)
     print(written.sum(), dev.max(), _cov_deviation(g, o, written))
     assert dev.max() < 1e-9
     assert _cov_deviation(g, o, written) < 1e-9
+
+
+# A field map with values that are not finite, or (FP64 form) whose differences
+# overflow FP32: the fit takes the trials, steps and statuses of the oracle,
+# which widens every value.
+@pytest.mark.parametrize("values, precision", [((np.nan,), 0), ((np.nan,), 1), ((np.inf,), 0), ((np.inf,), 1),
+                                               ((3e38, -3e38), 0)])
+@pytest.mark.parametrize("n", [200, 4000])
+def test_map_values_that_are_not_finite(kf, orc, values, precision, n):
+    tel = kf.make_telescope(n, seed=82, n_planes=8, field_map=True, field_n=21)
+    g = tel.field_grid.reshape(21, 21, 21, 4)
+    for k, v in enumerate(values):  # planes of the map in turn along x
+        g[:, :, 10 + k::len(values), 2] = v
+    cfg = kf.default_config(overstep_limit=0.1, precision=precision, max_rk_trials=40, max_steps=100)
+    o = orc.fit(tel, cfg, threads=0, variant="precise")
+    r = kf.fit_device(tel, cfg)
+    for k in ("status", "n_meas", "n_steps", "n_trials"):
+        assert np.array_equal(r[k], o[k]), k
