@@ -724,7 +724,7 @@ __device__ double chi2States(ZLane &L, const Params &P, const AdjParams &A, int6
       f0 = fma(-h0[c], E, f0);
       f1 = fma(-h1[c], E, f1);
     }
-    const double id = rcpFast(v00 * v11 - v01 * v01);
+    const double id = 1. / (v00 * v11 - v01 * v01); // (0 where large variances' product overflows)
     const double w0 = (v11 * f0 - v01 * f1) * id, w1 = (v00 * f1 - v01 * f0) * id;
     chi2 += f0 * w0 + f1 * w1;
     if (A.grad) {

@@ -74,3 +74,18 @@ def test_map_values_that_are_not_finite(kf, orc, values, precision, n):
     r = kf.fit_device(tel, cfg)
     for k in ("status", "n_meas", "n_steps", "n_trials"):
         assert np.array_equal(r[k], o[k]), k
+
+
+# A hit of huge variance says nothing, whether the product of its variances
+# overflows or not.
+def test_adjoint_of_hits_with_huge_variances(kf):
+    tel = kf.make_telescope(400, seed=83, n_planes=12, mis_shift=0.1, mis_rot=1e-3)
+    cfg = kf.default_config(overstep_limit=0.1)
+    tel.meas[3, 2], tel.meas[3, 4] = 1e150, 1e150
+    without = kf.AdjointBatch(tel, cfg).run(grad=True)
+    tel.meas[3, 2], tel.meas[3, 4] = 1e200, 1e200
+    g = kf.AdjointBatch(tel, cfg).run(grad=True)
+    assert np.all(g["status"] == 0) and np.all(without["status"] == 0)
+    for k in ("chi2", "grad_start", "grad_align", "grad_field_scale_track", "chi2_total"):
+        scale = np.max(np.abs(without[k]), axis=-1, keepdims=True)
+        assert np.max(np.abs(g[k] - without[k]) / np.where(scale > 0, scale, 1.)) < 1e-9, k
