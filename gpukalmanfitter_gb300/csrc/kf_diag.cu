@@ -1,8 +1,10 @@
-// kf_diag.cu — FP64 FMA throughput probe used as the roofline denominator.
+// kf_diag.cu — FP64 FMA throughput probe used as the roofline denominator, and
+// the fit kernels' reciprocals on given values.
 #include <cuda_runtime.h>
 
 #include "../../include/gb300kf.h"
 #include "../../include/gb300kf_diag.h"
+#include "kf_recip.cuh"
 
 namespace {
 
@@ -26,7 +28,21 @@ __global__ void __launch_bounds__(256) fmaChains(int iters, double seed) {
   if (r == 12345.678) g_sink[threadIdx.x] = r; // keeps the chains live
 }
 
+__global__ void __launch_bounds__(256) reciprocals(const double *a, int64_t n, double *rcp, double *rsqrt) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  rcp[i] = kfd::rcpFast(a[i]);
+  rsqrt[i] = kfd::rsqrtFast(a[i]);
+}
+
 } // namespace
+
+extern "C" int32_t kf_diag_reciprocals(const double *a, int64_t n, double *rcp, double *rsqrt, void *stream) {
+  if (n < 0 || n > (1LL << 30) || (n > 0 && (!a || !rcp || !rsqrt))) return KF_ERR_INVALID_ARGUMENT;
+  if (n == 0) return KF_SUCCESS;
+  reciprocals<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, n, rcp, rsqrt);
+  return cudaGetLastError() == cudaSuccess ? KF_SUCCESS : KF_ERR_CUDA;
+}
 
 extern "C" int32_t kf_diag_fp64_fma_rate(int32_t iters, double *gflops_out, void *stream) {
   if (!gflops_out || iters <= 0) return KF_ERR_INVALID_ARGUMENT;

@@ -53,6 +53,7 @@
 #pragma once
 
 #include "kf_device.cuh"
+#include "kf_recip.cuh"
 
 namespace kfd {
 
@@ -64,24 +65,6 @@ namespace kfd {
 enum FitForm { kUniform64 = 0, kGrid64 = 1, kMixed = 2, kUniformAny = 3, kMixedUniform = 4 };
 __host__ __device__ constexpr bool isMixed(int form) { return form == kMixed || form == kMixedUniform; }
 __host__ __device__ constexpr bool isUniform(int form) { return form == kUniform64 || form == kUniformAny; }
-
-// ---- FP64 reciprocal and reciprocal square root -----------------------------
-// The hardware's 20-bit estimate and one third-order step (Halley's family):
-// with e = 1 - a y, 1/a = y (1 + e + e^2 + ...), error e^3 < 2^-57.  Three
-// (four) FP64 instructions where the IEEE division's expansion takes nine.
-__device__ __forceinline__ double rcpFast(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a, y, 1.);
-  return fma(fma(e, e, e), y, y);
-}
-// with e = 1 - a y^2, 1/sqrt(a) = y (1 + e/2 + 3/8 e^2 + ...)
-__device__ __forceinline__ double rsqrtFast(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a * y, y, 1.);
-  return fma(fma(0.375, e, 0.5) * e, y, y);
-}
 
 // ---- shared-memory layout ---------------------------------------------------
 // One column per thread ([element][thread]).  Without process noise: F rows

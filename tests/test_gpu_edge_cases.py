@@ -89,3 +89,39 @@ def test_adjoint_of_hits_with_huge_variances(kf):
     for k in ("chi2", "grad_start", "grad_align", "grad_field_scale_track", "chi2_total"):
         scale = np.max(np.abs(without[k]), axis=-1, keepdims=True)
         assert np.max(np.abs(g[k] - without[k]) / np.where(scale > 0, scale, 1.)) < 1e-9, k
+
+
+def test_reciprocals_of_the_fit_kernels(kf):
+    """1 ulp and 2 ulp over many exponents and mantissas, from the error of the
+    method (kf_recip.cuh): a result of that error is off by less than 2 and 4
+    units of 2^-53 relative."""
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(5)
+    exps = np.concatenate([np.arange(-1000, 1001, 7), np.arange(-40, 41)])
+    a = (rng.uniform(1., 2., (exps.size, 2000)) * np.exp2(exps.astype(float))[:, None]).ravel()
+    a = np.concatenate([a, np.exp2(exps.astype(float)), np.nextafter(np.exp2(exps.astype(float)), 0.)])
+    d = torch.from_numpy(a).cuda()
+    r, s = torch.empty_like(d), torch.empty_like(d)
+    rc = kf.load().kf_diag_reciprocals(C.c_void_p(d.data_ptr()), C.c_int64(a.size), C.c_void_p(r.data_ptr()),
+                                       C.c_void_p(s.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    r, s = r.cpu().numpy(), s.cpu().numpy()
+    # 1 - a r and 1 - a s^2 in extended precision, exact enough to 2^-60; the
+    # exponents are split off first, so that nothing overflows
+    if np.finfo(np.longdouble).nmant >= 63:
+        wide = np.longdouble
+        er = np.abs(1 - wide(a) * wide(r)).astype(float)
+        m, e = np.frexp(a)
+        odd = (e & 1).astype(int)
+        m, e = np.ldexp(m, odd), e - odd
+        es = np.abs(1 - wide(m) * wide(np.ldexp(s, e // 2)) ** 2).astype(float) / 2
+        print(er.max() * 2 ** 53, es.max() * 2 ** 53)
+        assert er.max() < 2 * 2.0 ** -53 and es.max() < 4 * 2.0 ** -53
+    q = np.abs(r * a - 1.)
+    assert q.max() < 3 * 2.0 ** -53
+    special = torch.tensor([np.nan, np.inf, 0., 5e-324], dtype=torch.float64, device="cuda")
+    r, s = torch.empty_like(special), torch.empty_like(special)
+    kf.load().kf_diag_reciprocals(C.c_void_p(special.data_ptr()), C.c_int64(4), C.c_void_p(r.data_ptr()),
+                                  C.c_void_p(s.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert not np.isfinite(r.cpu().numpy()).any() and not np.isfinite(s.cpu().numpy()).any()
