@@ -1379,9 +1379,10 @@ __device__ __forceinline__ Gain gain(double S00, double S01, double S11, double 
   g.i1 = rcpFast(fma(-g.l, S01, S11));
   const double rp = fma(-g.l, r0, r1);
   g.e1 = rp * g.i1;
-  const double e0 = r0 * g.i0;
-  g.chi2 = fma(r0, e0, rp * g.e1);
-  g.e0 = fma(-g.l, g.e1, e0);
+  g.e0 = fma(-g.l, g.e1, r0 * g.i0);
+  // r S^-1 r as the reference forms it: with an infinite residual infinite or
+  // NaN as there (GainMatrixUpdater.hpp:84-93), which decides about an outlier
+  g.chi2 = fma(r0, g.e0, r1 * g.e1);
   return g;
 }
 

@@ -125,3 +125,22 @@ def test_reciprocals_of_the_fit_kernels(kf):
     kf.load().kf_diag_reciprocals(C.c_void_p(special.data_ptr()), C.c_int64(4), C.c_void_p(r.data_ptr()),
                                   C.c_void_p(s.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert not np.isfinite(r.cpu().numpy()).any() and not np.isfinite(s.cpu().numpy()).any()
+
+
+# A coordinate that is not finite: whether the hit is an outlier, and with it
+# the track's status, follows the reference's chi2 (infinite or NaN).
+@pytest.mark.parametrize("n", [500, 5000])
+@pytest.mark.parametrize("field_map", [False, True])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_coordinates_that_are_not_finite(kf, orc, n, field_map, precision, value):
+    tel = kf.make_telescope(n, seed=84, n_planes=10, hit_prob=0.9, field_map=field_map, field_n=21)
+    tel.meas[3, 1, ::2] = value
+    tel.meas[5, 0, ::3] = value
+    cfg = kf.default_config(overstep_limit=0.1, precision=precision, outlier_chi2_cut=25.0, max_rk_trials=40,
+                            max_steps=100)
+    o = orc.fit(tel, cfg, threads=0, variant="precise")
+    g = kf.fit_device(tel, cfg)
+    assert len(np.unique(o["status"])) > 1
+    for k in ("status", "n_meas"):
+        assert np.array_equal(g[k], o[k]), k
