@@ -150,7 +150,10 @@ int32_t enqueueBatched(Params &P, const kf_config_t *cfg, char *base, const Batc
   q.hist = reinterpret_cast<int32_t *>(base + L.hist);
   q.offs = reinterpret_cast<int32_t *>(base + L.offs);
   q.counter = reinterpret_cast<int32_t *>(base + L.counter);
-  return launchFit(P, cfg->precision, cfg->block_size, cfg->min_blocks_per_sm, q, s);
+  // with material effects the shape fields say nothing (prepare), whether the
+  // geometry has material or not
+  const bool shape = !cfg->material_effects;
+  return launchFit(P, cfg->precision, shape ? cfg->block_size : 0, shape ? cfg->min_blocks_per_sm : 0, q, s);
 }
 
 int32_t prepare(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t *cfg,

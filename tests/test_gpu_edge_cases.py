@@ -144,3 +144,33 @@ def test_coordinates_that_are_not_finite(kf, orc, n, field_map, precision, value
     assert len(np.unique(o["status"])) > 1
     for k in ("status", "n_meas"):
         assert np.array_equal(g[k], o[k]), k
+
+
+# With material effects the batched form takes no notice of the launch shape
+# fields, whatever they hold, on a geometry with material or without.
+@pytest.mark.parametrize("shape", [(256, 0), (256, 4), (128, 1), (0, 1), (96, 7)])
+@pytest.mark.parametrize("material, smoothed", [(0.3, False), (0.3, True), (0., False)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_material_ignores_the_launch_shape(kf, shape, material, smoothed, precision):
+    import torch
+    tel = kf.make_telescope(2500, seed=85, n_planes=8)
+    tel.material = np.tile(kf.silicon(material), (8, 1)) if material else None
+    opt = dict(overstep_limit=0.1, precision=precision, material_effects=3)
+    b = kf.DeviceBatch(tel, kf.default_config(**opt), smoothed=smoothed)
+    b.fit_sorted()
+    ref = b.results()
+    b = kf.DeviceBatch(tel, kf.default_config(block_size=shape[0], min_blocks_per_sm=shape[1], **opt),
+                       smoothed=smoothed)
+    b.fit_sorted()
+    g = b.results()
+    s = torch.cuda.Stream()
+    b.make_plan(s)
+    for v in b.out.values():
+        v.fill_(3)
+    s.wait_stream(torch.cuda.current_stream())
+    b.launch_plan(s)
+    s.synchronize()
+    p = b.results()
+    assert np.all(ref["status"] == 0)
+    for k, v in ref.items():
+        assert np.array_equal(g[k], v) and np.array_equal(p[k], v), k
