@@ -150,6 +150,7 @@ int32_t enqueueBatched(Params &P, const kf_config_t *cfg, char *base, const Batc
   q.hist = reinterpret_cast<int32_t *>(base + L.hist);
   q.offs = reinterpret_cast<int32_t *>(base + L.offs);
   q.counter = reinterpret_cast<int32_t *>(base + L.counter);
+  q.apart = true;
   // with material effects the shape fields say nothing (prepare), whether the
   // geometry has material or not
   const bool shape = !cfg->material_effects;

@@ -216,7 +216,7 @@ int32_t kf_fit_batch(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t
   // it does not fit
   int32_t *w = reinterpret_cast<int32_t *>(static_cast<double *>(workspace) + 35 * P.wsStride);
   int32_t *v = reinterpret_cast<int32_t *>(static_cast<double *>(workspace) + 36 * P.wsStride);
-  const QueueBuffers q = {w, v, v + kSortBuckets, v + 2 * kSortBuckets};
+  const QueueBuffers q = {w, v, v + kSortBuckets, v + 2 * kSortBuckets, false};
   return launchFit(P, cfg->precision, 0, 0, q, static_cast<cudaStream_t>(stream));
 }
 

@@ -2277,4 +2277,17 @@ __device__ void initLane(Lane<R, H> &L, const Params &P, const PlaneD *planes, i
   navStatus(L, P, planes);
 }
 
+// blocks: what the batch needs; left at no more than the device holds at once
+template <class K>
+inline cudaError_t residentBlocks(K *kernel, int threads, size_t smem, int64_t &blocks) {
+  int dev = 0, sms = 0, per = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
+  if (e != cudaSuccess) return e;
+  const int64_t most = (int64_t)sms * (per > 0 ? per : 1);
+  if (blocks > most) blocks = most;
+  return cudaSuccess;
+}
+
 } // namespace kfd

@@ -37,9 +37,11 @@ int32_t checkCommon(const kf_inputs_t *in, const kf_config_t *cfg, const kf_geom
 constexpr int kSortBuckets = 2048;
 int32_t sortQueue(const kfd::Params &P, int32_t *hist, int32_t *offs, int32_t *perm,
                   int32_t *counter, cudaStream_t s);
-// device memory for it: perm of n, hist and offs of kSortBuckets ints, one counter
+// device memory for it: perm of n, hist and offs of kSortBuckets ints, one
+// counter; apart: in memory of their own, not among the states' records
 struct QueueBuffers {
   int32_t *perm, *hist, *offs, *counter;
+  bool apart;
 };
 // compiled launch shapes (threads per block, blocks per SM) of the batched
 // form: the index-th (the first is the default); whether a request (0: the

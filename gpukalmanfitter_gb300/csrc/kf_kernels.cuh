@@ -151,15 +151,8 @@ template <int FORM> __global__ void __launch_bounds__(32, 8) fitCoop(const __gri
     const int64_t need = (P.n + per_block - 1) / per_block;                                  \
     int64_t blocks = need;                                                                   \
     if (P.queueCounter && !P.split) {                                                        \
-      int dev = 0, sms = 0, per = 0;                                                         \
-      e = cudaGetDevice(&dev);                                                               \
+      e = kfd::residentBlocks(kernel, bs, smem, blocks);                                     \
       if (e != cudaSuccess) return e;                                                        \
-      e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);                 \
-      if (e != cudaSuccess) return e;                                                        \
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, bs, smem);             \
-      if (e != cudaSuccess) return e;                                                        \
-      blocks = (int64_t)sms * (per > 0 ? per : 1);                                           \
-      if (blocks > need) blocks = need;                                                      \
     }                                                                                        \
     if (blocks < 1) blocks = 1;                                                              \
     kernel<<<(unsigned)blocks, bs, smem, s>>>(P);                                            \

@@ -157,6 +157,12 @@ int32_t launchFit(Params &P, int precision, int bs, int minb, const QueueBuffers
   P.lanes = 32;
   P.split = 0;
   if (P.materialEffects && P.oSmoothed) {
+    if (q.apart) { // (this form's records leave no words for the plain call to sort in)
+      const int32_t rc = sortQueue(P, q.hist, q.offs, q.perm, q.counter, s);
+      if (rc) return rc;
+      P.perm = q.perm;
+      P.queueCounter = q.counter;
+    }
     e = (mixed ? launchFitMaterialStates_mixed : launchFitMaterialStates_fp64)(P, 0, s);
     return e == cudaSuccess ? KF_SUCCESS : cudaFail(e, "fit kernel launch");
   }

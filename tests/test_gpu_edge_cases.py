@@ -174,3 +174,32 @@ def test_material_ignores_the_launch_shape(kf, shape, material, smoothed, precis
     assert np.all(ref["status"] == 0)
     for k, v in ref.items():
         assert np.array_equal(g[k], v) and np.array_equal(p[k], v), k
+
+
+def _queue_order(kf, b):
+    """The order in the batched form's workspace (behind the states' records)."""
+    import ctypes as C
+    at = -(-kf.load().kf_workspace_size(C.byref(b.cfg), b.tel.n, b.tel.n_surfaces) // 256) * 256
+    return b.ws[at:at + 4 * b.tel.n].view(dtype=__import__("torch").int32).cpu().numpy()
+
+
+# Material with smoothed states: the batched form fits its tracks in the order
+# of their lengths, below and above what the device holds at once, with the
+# results of the plain form.
+@pytest.mark.parametrize("n", [700, 80_000])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_material_with_states_runs_in_order_of_length(kf, n, precision):
+    tel = kf.make_telescope(n, seed=86, n_planes=8, min_len=3, max_len=8, hit_prob=0.9)
+    tel.material = np.tile(kf.silicon(0.3), (8, 1))
+    b = kf.DeviceBatch(tel, kf.default_config(overstep_limit=0.1, material_effects=3, precision=precision),
+                       smoothed=True)
+    b.fit()
+    ref = b.results()
+    b.ws.zero_()
+    b.fit_sorted()
+    g = b.results()
+    for k, v in ref.items():
+        assert np.array_equal(g[k], v), k
+    order = _queue_order(kf, b)
+    assert np.array_equal(np.sort(order), np.arange(n))
+    assert np.all(np.diff(tel.n_planes[order]) <= 0)
