@@ -276,8 +276,10 @@ int32_t kf_autotune(const kf_inputs_t *in, kf_outputs_t *out, const kf_config_t 
   kf_config_t bestCfg = *cfg;
   int32_t rc = KF_SUCCESS;
   int bs = 0, minb = 0;
-  // with material effects there is one shape
-  for (int v = 0; fitShape(v, &bs, &minb) && (v == 0 || !cfg->material_effects); ++v) {
+  // the library's own launch first, where it is none of the shapes; with
+  // material effects there is one shape
+  const bool own = !cfg->material_effects && !launchesAShape(sample.n_tracks);
+  for (int v = own ? -1 : 0; v < 0 || (fitShape(v, &bs, &minb) && (v == 0 || !cfg->material_effects)); ++v) {
     kf_config_t c = *cfg;
     c.kernel = KF_KERNEL_PERSISTENT;
     c.block_size = bs;

@@ -44,8 +44,10 @@ struct QueueBuffers {
   bool apart;
 };
 // compiled launch shapes (threads per block, blocks per SM) of the batched
-// form: the index-th (the first is the default); whether a request (0: the
-// default) is one of them
+// form: the index-th; whether a request (0, 0: the library's choice) is one of
+// them; whether the library's choice for n tracks is one of them (256 x 1, a
+// queue) and not a launch of its own for fewer tracks
+bool launchesAShape(int64_t n);
 bool fitShape(int index, int *bs, int *minb);
 bool shapeCompiled(int bs, int minb);
 // enqueue the fit of P on s: sort and fit kernel.  The shape (0, 0: chosen

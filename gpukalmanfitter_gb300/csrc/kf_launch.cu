@@ -47,7 +47,9 @@ struct Shape {
   int bs, minb;
   const Budget *budget;
 };
-// (threads per block, blocks per SM); the first is the default
+// (threads per block, blocks per SM: the register budget that the kernel is
+// compiled for; shared memory may hold fewer, of 128 x 5 four).  The first
+// gives the budget of the library's own launches.
 const Shape kShapes[] = {
     {128, 2, &kBudget255}, {64, 4, &kBudget255},  {256, 1, &kBudget255}, {128, 3, &kBudget168},
     {128, 4, &kBudget128}, {64, 8, &kBudget128},  {256, 2, &kBudget128}, {128, 5, &kBudget96},
@@ -66,7 +68,7 @@ bool fitShape(int index, int *bs, int *minb) {
   return true;
 }
 
-// the shape for a request: the default for (0, 0), else 0 stands for 128
+// the shape for a request: the first for (0, 0), else 0 stands for 128
 // threads and for 4 blocks per SM
 static const Shape *findShape(int bs, int minb) {
   if (!bs && !minb) return &kShapes[0];
@@ -141,6 +143,14 @@ static Spread spread(int64_t n, int sms) {
   if (perSm > 8) return {32, room, room};
   const int lanes = (int)((n + sms * perSm - 1) / (sms * perSm));
   return {lanes, room && lanes >= 8, false};
+}
+
+bool launchesAShape(int64_t n) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return true;
+  return spread(n, sms).queue;
 }
 
 // Batches of up to kCoopMost tracks an SM run eight lanes a track, again as few

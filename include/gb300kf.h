@@ -122,7 +122,9 @@ typedef struct kf_config {
   int32_t min_blocks_per_sm; /* batched form: CTAs per SM the kernel is compiled
                                 for (its register budget), 0 alone = 4; shapes
                                 (threads x CTAs): 128 x 2..5, 64 x 4, 64 x 8,
-                                256 x 1, 256 x 2; kf_autotune picks one */
+                                256 x 1, 256 x 2; shared memory may hold fewer
+                                CTAs (of 128 x 5 four); kf_autotune picks one,
+                                or the library's choice */
   int32_t material_effects;  /* bit 0: multiple scattering, bit 1: energy loss
                                 at the surfaces' material (kf_geometry_t.material)
                                 after each filter update (KalmanFitter.hpp:405-449,
@@ -286,12 +288,14 @@ int32_t kf_batch_plan_create(kf_batch_plan_t **plan, const kf_inputs_t *in,
 int32_t kf_batch_plan_launch(kf_batch_plan_t *plan, void *stream);
 void kf_batch_plan_destroy(kf_batch_plan_t *plan);
 
-/* Times every compiled kernel shape (threads per CTA and CTAs per
- * SM, see kf_config_t.min_blocks_per_sm) of cfg->precision on the first min(n, 524288) tracks of the batch
- * (best of three runs after a warm-up) and returns the fastest configuration
- * in *tuned (and its time per fit of the sample in *best_ms).  Overwrites
- * the outputs of those tracks.  Shapes differ in register allocation only;
- * results agree to rounding (not bitwise) across shapes. */
+/* Times every compiled kernel shape (threads per CTA and CTAs per SM, see
+ * kf_config_t.min_blocks_per_sm) of cfg->precision on the first
+ * min(n, 524288) tracks of the batch, and for batches of up to 256 tracks an SM
+ * the library's own launch too, which is none of the shapes there (best of
+ * three runs after a warm-up).  Returns the fastest configuration in *tuned
+ * (both shape fields 0: the library's choice) and its time per fit of the
+ * sample in *best_ms.  Overwrites the outputs of those tracks.  Results agree
+ * to rounding (not bitwise) across shapes. */
 int32_t kf_autotune(const kf_inputs_t *in, kf_outputs_t *out,
                     const kf_config_t *cfg, const kf_geometry_t *geo,
                     const kf_field_t *field, void *workspace,

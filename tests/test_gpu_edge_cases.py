@@ -203,3 +203,34 @@ def test_material_with_states_runs_in_order_of_length(kf, n, precision):
     order = _queue_order(kf, b)
     assert np.array_equal(np.sort(order), np.arange(n))
     assert np.all(np.diff(tel.n_planes[order]) <= 0)
+
+
+# The autotuner's choice is no slower than the library's own launch, which runs
+# small batches in a way that no launch shape does.  (10 %: what two timings of
+# one kernel may differ by.)
+@pytest.mark.parametrize("n", [1000, 3000, 20_000])
+def test_autotune_of_small_batches(kf, n):
+    import torch
+    tel = kf.make_telescope(n, seed=87)
+    b = kf.DeviceBatch(tel, kf.default_config(overstep_limit=0.1))
+
+    def least_time():
+        times = []
+        for _ in range(20):
+            e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e[0].record()
+            b.fit_sorted()
+            e[1].record()
+            e[1].synchronize()
+            times.append(e[0].elapsed_time(e[1]))
+        return min(times[3:])
+
+    b.fit_sorted()
+    ref = b.results()
+    own = least_time()
+    tuned, ms = b.autotune()
+    best = least_time()
+    print(n, own, best, ms, tuned.block_size, tuned.min_blocks_per_sm)
+    assert ms > 0 and best <= 1.1 * own
+    g = b.results()
+    assert np.array_equal(g["status"], ref["status"]) and np.array_equal(g["n_steps"], ref["n_steps"])
