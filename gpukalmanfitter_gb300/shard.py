@@ -18,13 +18,16 @@ CHUNK = 32  # tracks per warp of the persistent kernel
 
 
 def work_keys(n_planes: np.ndarray | None, start_qop: np.ndarray, n_surfaces: int) -> np.ndarray:
-    """Ascending key = descending expected work (the batched form's queue key)."""
-    L = np.full(start_qop.shape, n_surfaces) if n_planes is None else np.clip(n_planes, 0, n_surfaces)
-    q = np.abs(start_qop)
-    with np.errstate(divide="ignore", invalid="ignore"):
-        qb = np.where((q > 0) & np.isfinite(q), np.floor((np.log2(q) + 7.0) * 2.0), 0)
-    qb = np.clip(qb, 0, 15).astype(np.int64)
-    return (64 - L.astype(np.int64)) * 16 + (15 - qb)
+    """Ascending key = descending expected work: the batched form's queue key
+    (workKey of csrc/kf_batch.cu): sequence length, then |q/p| in quarter
+    octaves."""
+    L = np.full(start_qop.shape, n_surfaces) if n_planes is None else n_planes
+    L = np.clip(L, 1, n_surfaces).astype(np.int64)
+    with np.errstate(divide="ignore", invalid="ignore", over="ignore"):
+        q = np.abs(start_qop).astype(np.float32)
+        bins = np.floor((np.log2(q) + np.float32(7)) * np.float32(4))
+    qb = np.where((q > 0) & (q < np.float32(3.0e38)), np.clip(bins, 0, 31), 0).astype(np.int64)
+    return (64 - L) * 32 + (31 - qb)
 
 
 def balanced_ranges(keys: np.ndarray, world: int, chunk: int = CHUNK) -> list[np.ndarray]:
