@@ -80,8 +80,10 @@ __host__ __device__ constexpr int u5(int i, int j) { // upper triangle of 5x5
 }
 
 // a state's record in the workspace: x_p - F D (6), F rows 0-3 (20), F's time
-// row (5), and for the first state the direction's trigonometry (4)
-enum { kRecX = 0, kRecF = 6, kRecT = 26, kRecTrig = 31 };
+// row (5), and for the first state the direction's trigonometry (4) and, once
+// its x is read, in place of phi the time's q/p factor that the leg to the line
+// owes to an earlier momentum
+enum { kRecX = 0, kRecRest = 2, kRecF = 6, kRecT = 26, kRecTrig = 31 };
 static_assert(kRecTrig + 4 <= kStateStride, "state record");
 
 template <int FORM, int GROUP = 1> struct LegState;
@@ -1748,6 +1750,14 @@ __device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT, H> &L, const P
 #pragma unroll
     for (int r = 0; r < 4; ++r) x[r] += L.D(r);
   }
+  // the time's q/p factor of a leg that has begun: its own momentum's (d37 is
+  // kept up only where a surface's Jacobian has a time row)
+  double d37 = 0.;
+  if (L.stepped) {
+    const double m = P.mass * L.qop;
+    d37 = P.mass * m * rsqrtFast(fma(m, m, 1.));
+    if constexpr (isMixed(FORM)) L.Jb += (float)(L.sTr * (d37 - (double)L.d37f));
+  }
   const PlaneD &pl = planes[L.firstPlane];
   updateState(L, P, pl, x[0], x[1], t, x[2], x[3], qop, true);
   if (!P.faithful) {
@@ -1761,6 +1771,7 @@ __device__ __forceinline__ bool finalizeSmooth(FitLane<FORM, MAT, H> &L, const P
     }
   }
   // (a leg that had begun when the track ran out of planes goes on)
+  if constexpr (!isMixed(FORM)) *recPtr(P, L, 0, kRecRest) = L.stepped ? legPath(L) * (d37 - L.d37) : 0.;
   L.t = fma(-legPath(L), L.dtds, tm);
   L.navDir = -1;
   ssInit(L, -1. * DBL_MAX);
@@ -1812,6 +1823,7 @@ __device__ __forceinline__ void reachPerigee(FitLane<FORM, MAT, H> &L, const Par
     toFrame<LT>(P, sp, fs);
     toFrame<LT>(P, sv, fv);
     boundRows<true>(L, P, planes, tl, 0., fX, fY, fs, fv, f0, f1, true, J, J5);
+    J5[4] += *recPtr(P, L, 0, kRecRest); // (boundRows gives all of the leg the last momentum)
     if constexpr (MAT) {
       sandwich(J, J5, C, Ct, cov);
     } else {

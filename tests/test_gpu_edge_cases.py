@@ -234,3 +234,26 @@ def test_autotune_of_small_batches(kf, n):
     assert ms > 0 and best <= 1.1 * own
     g = b.results()
     assert np.array_equal(g["status"], ref["status"]) and np.array_equal(g["n_steps"], ref["n_steps"])
+
+
+# Such tracks against the oracle: the leg that had begun keeps the time's q/p
+# derivative of its own momentum, also where the smoothed one differs (low
+# momenta, energy loss).
+@pytest.mark.parametrize("n", [2000, 4000])
+@pytest.mark.parametrize("field_map", [False, True])
+@pytest.mark.parametrize("material", [0., 0.3])
+def test_time_of_tracks_that_miss_their_last_planes(kf, orc, n, field_map, material):
+    tel = kf.make_telescope(n, seed=88, n_planes=15, x_first=80., x_step=80., min_len=5, max_len=15, hit_prob=0.9,
+                            p_min=0.3, p_max=1.5, bz_tesla=0.3)
+    tel.material = np.tile(kf.silicon(material), (15, 1)) if material else None
+    if field_map:
+        tel = _in_constant_map(tel, kf)
+    cfg = kf.default_config(overstep_limit=0.01, material_effects=3 if material else 0)
+    o = orc.fit(tel, cfg, threads=0, variant="precise")
+    g = kf.fit_device(tel, cfg)
+    for k in ("status", "n_meas", "n_steps"):
+        assert np.array_equal(g[k], o[k]), k
+    written = (o["cov"][0] != 0.) & (o["status"] != 0)
+    print(written.sum(), _cov_deviation(g, o, written))
+    assert written.sum() > 20
+    assert _cov_deviation(g, o, written) < 1e-9
