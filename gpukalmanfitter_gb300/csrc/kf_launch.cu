@@ -87,8 +87,12 @@ static void toFieldFrame(Params &P) {
   P.rotated = B[0] != 0. || B[1] != 0.;
   P.Bz = B[2];
   if (!P.rotated) return;
-  const double n = std::sqrt(B[0] * B[0] + B[1] * B[1] + B[2] * B[2]);
-  const double z[3] = {B[0] / n, B[1] / n, B[2] / n};
+  // (by a power of two to about 1, so that no square leaves the range)
+  const double big = std::fmax(std::fabs(B[0]), std::fmax(std::fabs(B[1]), std::fabs(B[2])));
+  const int e = std::isfinite(big) ? std::ilogb(big) : 0;
+  const double b[3] = {std::scalbn(B[0], -e), std::scalbn(B[1], -e), std::scalbn(B[2], -e)};
+  const double n = std::sqrt(b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
+  const double z[3] = {b[0] / n, b[1] / n, b[2] / n};
   // x axis: the coordinate axis least along z, made orthogonal to it
   int a = 0;
   for (int i = 1; i < 3; ++i)
@@ -103,7 +107,7 @@ static void toFieldFrame(Params &P) {
     P.rot[3 + i] = y[i];
     P.rot[6 + i] = z[i];
   }
-  P.Bz = n;
+  P.Bz = std::scalbn(n, e);
   auto turn = [&](double v[3]) {
     double o[3];
     for (int i = 0; i < 3; ++i)

@@ -257,3 +257,27 @@ def test_time_of_tracks_that_miss_their_last_planes(kf, orc, n, field_map, mater
     print(written.sum(), _cov_deviation(g, o, written))
     assert written.sum() > 20
     assert _cov_deviation(g, o, written) < 1e-9
+
+
+# A uniform field too weak to square has no say, whatever its direction.
+@pytest.mark.parametrize("tesla", [(1e-170, 0., 0.), (1e-170, 1e-172, -1e-171)])
+@pytest.mark.parametrize("n", [100, 4000])
+def test_vanishing_field_off_axis(kf, tesla, n):
+    tel = kf.make_telescope(n, seed=94, n_planes=8, bz_tesla=0.)
+    cfg = kf.default_config(overstep_limit=0.1)
+    ref = kf.fit_device(tel, cfg)
+    along_z = tel.field
+
+    def field(grid_ptr=None, scale=1.0):
+        f = along_z(grid_ptr, scale)
+        for a in range(3):
+            f.value[a] = tesla[a] * kf.TESLA
+        return f
+
+    tel.field = field
+    g = kf.fit_device(tel, cfg)
+    assert np.all(ref["status"] == 0)
+    for k in ("status", "n_meas", "n_steps", "n_trials"):
+        assert np.array_equal(g[k], ref[k]), k
+    sig = np.sqrt(np.abs(ref["cov"][[0, 6, 11, 15, 18, 20]]))
+    assert np.max(np.abs(g["params"] - ref["params"]) / np.maximum(np.abs(ref["params"]), sig)) < 1e-9
