@@ -9,8 +9,8 @@
 // G_j = sum over k <= j of dchi2/dE_k that each hit's dl receives.  The time
 // is part of no measurement and does not occur.
 //
-// A. forward: the fit's lane, whose hook stores per state (F, C0, D before the
-//    update, the predicted state, the leg's transport scalars; 70 words) and
+// A. forward: the fit's lane, whose hook stores per state (F, C0, the update
+//    dl, the predicted state, the leg's transport scalars; 70 words) and
 //    tapes the RK steps and step constraints (13 and 2 words) and per hit the
 //    Jacobian, C0 h and the gain (36);
 // B. chi2 and sum of dchi2/dE over the states;
@@ -36,7 +36,7 @@ namespace adj {
 // a state's record: word e in P.ws (e < 37) or A.stateBar
 enum {
   zH = 0,     // F rows 0, 1 (10)
-  zD = 10,    // D before the update (5)
+  zD = 10,    // the update's dl, later the sum G (5)
   zX = 15,    // predicted loc0, loc1
   zF2 = 17,   // F rows 2, 3 (10)
   zC = 27,    // C0 before the update (15)
@@ -121,7 +121,6 @@ struct ZHook {
     for (int c = 0; c < 5; ++c) {
       word(zH + c, L.F(0, c));
       word(zH + 5 + c, L.F(1, c));
-      word(zD + c, L.D(c));
     }
     word(zX, x0);
     word(zX + 1, x1);
@@ -163,6 +162,8 @@ struct ZHook {
       for (int c = 0; c < 5; ++c) put(J[r][c]);
   }
   __device__ __forceinline__ void update(const double (&w0)[5], const double (&w1)[5], const Gain &g) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) word(zD + c, fma(w0[c], g.e0, w1[c] * g.e1));
     if (!rec) return;
 #pragma unroll
     for (int c = 0; c < 5; ++c) put(w0[c]);
@@ -190,7 +191,7 @@ using ZLane = FitLane<kUniform64, false, ZHook>;
 // ---- the running adjoint ----------------------------------------------------
 // In the lane's shared-memory column, once the forward pass is done: F(r, c)
 // and C0(e) hold the adjoints of F and of C0 (B: the symmetric matrix, off-
-// diagonal entries halved), D the final D, Ct(c) the sum G.
+// diagonal entries halved), D(c) the sum E of the updates passed so far.
 struct ZAdj {
   double pos[3], dir[3], qop, Bz;
   double g, b, r, q1, s, c0, c1, a0, a1; // leg scalars
@@ -369,19 +370,16 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
     for (int e = 0; e < 15; ++e) C[e] = rec(s, zC + e);
     // chi2's own term
     const double p0 = rec(s, zRho), p1 = rec(s, zRho + 1);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      const double E = L.D(c) - rec(s, zD + c);
-      L.F(0, c) = fma(-p0, E, L.F(0, c));
-      L.F(1, c) = fma(-p1, E, L.F(1, c));
-      w0[c] = Jt[tW + c];
-      w1[c] = Jt[tW + 5 + c];
-    }
     const Gain g = {Jt[tGain], Jt[tGain + 1], Jt[tGain + 2], Jt[tGain + 3], Jt[tGain + 4], 0.};
     double dl[5], D0 = 0., D1 = 0.; // h . dl: the shift of the predicted position
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
+      w0[c] = Jt[tW + c];
+      w1[c] = Jt[tW + 5 + c];
       dl[c] = fma(w0[c], g.e0, w1[c] * g.e1);
+      const double E = L.D(c) += dl[c];
+      L.F(0, c) = fma(-p0, E, L.F(0, c));
+      L.F(1, c) = fma(-p1, E, L.F(1, c));
       D0 = fma(h0[c], dl[c], D0);
       D1 = fma(h1[c], dl[c], D1);
     }
@@ -408,9 +406,7 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
       const double f2 = rec(s, zF2 + c), f3 = rec(s, zF2 + 5 + c);
-      const double Gc = L.Ct(c);
-      dlb[c] = Gc + ph1 * f2 + th1 * f3 + X0b * h0[c] + X1b * h1[c] + (c == 4 ? qopb : 0.);
-      L.Ct(c) = Gc + p0 * h0[c] + p1 * h1[c]; // less this state's dchi2/dE
+      dlb[c] = rec(s, zD + c) + ph1 * f2 + th1 * f3 + X0b * h0[c] + X1b * h1[c] + (c == 4 ? qopb : 0.);
       L.F(2, c) = fma(ph1, dl[c], L.F(2, c));
       L.F(3, c) = fma(th1, dl[c], L.F(3, c));
     }
@@ -703,26 +699,25 @@ __device__ void reverseEvent(TapeRef Jt, int s, ZAdj &R, ZLane &L, const Params 
   R.dir[2] += thb * f1[2];
 }
 
-// chi2 of a track with ns states, the sum of dchi2/dE into Ct, and with grad
-// each state's 2 V^-1 rho into its record
-__device__ double chi2States(ZLane &L, const Params &P, const AdjParams &A, int64_t u, int64_t i,
-                             int ns) {
+// chi2 of a track with ns states, backwards with the sum E of the updates; with
+// grad each state's 2 V^-1 rho into its record, and then, forwards, the sum G
+// of dchi2/dE in place of its update (sums of their own: differences of running
+// sums cancel)
+__device__ double chi2States(const Params &P, const AdjParams &A, int64_t u, int64_t i, int ns) {
   const int64_t n = P.n;
-  double chi2 = 0., G[5] = {0., 0., 0., 0., 0.};
-  for (int s = 0; s < ns; ++s) {
+  double chi2 = 0., E[5] = {0., 0., 0., 0., 0.};
+  for (int s = ns - 1; s >= 0; --s) {
     const int inf = A.info[(int64_t)s * n + u];
     if (inf & 256) continue;
     const double *rc = P.ws + (int64_t)s * kStateStride * n + u;
     const double *mp = P.meas + (size_t)(inf & 255) * 5 * P.stride + i;
     const double v00 = mp[2 * P.stride], v01 = mp[3 * P.stride], v11 = mp[4 * P.stride];
-    double f0 = mp[0] - rc[zX * n], f1 = mp[P.stride] - rc[(zX + 1) * n], h0[5], h1[5];
+    double f0 = mp[0] - rc[zX * n], f1 = mp[P.stride] - rc[(zX + 1) * n];
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-      const double E = L.D(c) - rc[(zD + c) * n];
-      h0[c] = rc[(zH + c) * n];
-      h1[c] = rc[(zH + 5 + c) * n];
-      f0 = fma(-h0[c], E, f0);
-      f1 = fma(-h1[c], E, f1);
+      E[c] += rc[(zD + c) * n];
+      f0 = fma(-rc[(zH + c) * n], E[c], f0);
+      f1 = fma(-rc[(zH + 5 + c) * n], E[c], f1);
     }
     const double id = 1. / (v00 * v11 - v01 * v01); // (0 where large variances' product overflows)
     const double w0 = (v11 * f0 - v01 * f1) * id, w1 = (v00 * f1 - v01 * f0) * id;
@@ -732,11 +727,20 @@ __device__ double chi2States(ZLane &L, const Params &P, const AdjParams &A, int6
       rb[0] = 2. * w0;
       rb[n] = 2. * w1;
     }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) G[c] -= 2. * (w0 * h0[c] + w1 * h1[c]);
   }
+  if (!A.grad) return chi2;
+  double G[5] = {0., 0., 0., 0., 0.};
+  for (int s = 0; s < ns; ++s) {
+    if (A.info[(int64_t)s * n + u] & 256) continue;
+    double *rc = P.ws + (int64_t)s * kStateStride * n + u;
+    const double *rb = A.stateBar + ((int64_t)s * kStateStride + zRho - kStateStride) * n + u;
+    const double p0 = rb[0], p1 = rb[n];
 #pragma unroll
-  for (int c = 0; c < 5; ++c) L.Ct(c) = G[c];
+    for (int c = 0; c < 5; ++c) {
+      G[c] -= p0 * rc[(zH + c) * n] + p1 * rc[(zH + 5 + c) * n];
+      rc[(zD + c) * n] = G[c];
+    }
+  }
   return chi2;
 }
 
@@ -788,7 +792,7 @@ __global__ void __launch_bounds__(kZBlock, 8) adjointZ(const __grid_constant__ P
   if (valid) A.status[i] = left ? kLeft : (ok && L.hook.full ? KF_TRACK_ADJOINT_FAILED : L.status);
   ok = ok && !left && !L.hook.full;
   // ---- B
-  if (ok) A.chi2[i] = chi2States(L, P, A, u, i, ns);
+  if (ok) A.chi2[i] = chi2States(P, A, u, i, ns);
   if (!A.grad) return;
   // ---- C
   ZAdj R;
@@ -800,6 +804,7 @@ __global__ void __launch_bounds__(kZBlock, 8) adjointZ(const __grid_constant__ P
   for (int r = 0; r < 4; ++r)
     for (int c = 0; c < 5; ++c) L.F(r, c) = 0.;
   for (int e = 0; e < 15; ++e) L.C0(e) = 0.;
+  for (int c = 0; c < 5; ++c) L.D(c) = 0.;
   const TapeRef tape = {L.hook.tape, P.n};
   int top = ok ? L.hook.top : 0, state = ns;
   const double q = L.q;
