@@ -35,8 +35,10 @@ int32_t cudaFail(cudaError_t e, const char *where) {
 }
 
 size_t wsBytes(int64_t n, int32_t nSurf, bool material) {
-  // per state: predicted and filtered parameters and the Jacobian; with
-  // material also the predicted and filtered covariance (general smoother)
+  // per state kStateStride words: the plain fits use the first state's (its
+  // parameters and Jacobian onto the start frame, and the queue's arrays in the
+  // last two), with smoothed states all of them; with material also room for
+  // the predicted and filtered covariance (the smoother of returned states)
   return (size_t)nSurf * (kStateStride + (material ? 42 : 0)) * (size_t)n * sizeof(double);
 }
 

@@ -29,7 +29,9 @@
 // so the result is the reference's algebra with a different rounding order.
 //
 // Precision.  Lane<R> carries the transport Jacobians in R.  R = double is
-// the plain form (FP64 throughout).  R = float is the mixed form: field
+// FP64 throughout.  R = float is the mixed precision of the fits with material
+// whose smoothed states are returned (kf_fit.cuh's mixed forms have the same
+// stages, transport and decisions and no covariance per plane): field
 // interpolation in FP32 on differences from a cell corner, RK4 stages k2..k4
 // as FP32 offsets from an FP64 k1, the error estimate, the transport matrix
 // and all Jacobians in FP32; position, direction, time, step sizes,
@@ -52,7 +54,8 @@
 namespace kfd {
 
 constexpr int kStateStride = 37; // doubles per stored measurement state
-// layout of one stored state (smoother input):
+// layout of one stored state of Lane<R> (smoother input; kf_fit.cuh and
+// kf_adjoint_z.cu lay out their own records in as many words):
 //   [0,6) predicted params, [6,12) filtered params, [12,37) bound-to-bound
 //   jacobian from the previous state: rows 0..3 cols 0..4 (20) and row 5
 //   cols 0..4 (5); the other entries are structural (row 4 = e4, column

@@ -40,8 +40,6 @@ __device__ __forceinline__ ff twoProd(float a, float b) {
   return {p, __fmaf_rn(a, b, -p)};
 }
 
-__device__ __forceinline__ double join(ff x) { return (double)x.hi + (double)x.lo; }
-
 // pair product (error a few 2^-44 relative)
 __device__ __forceinline__ ff mul(ff x, ff y) {
   const ff p = twoProd(x.hi, y.hi);

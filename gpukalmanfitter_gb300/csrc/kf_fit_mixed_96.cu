@@ -1,5 +1,5 @@
 // kf_fit_mixed_96.cu — mixed fit kernels with up to 96 registers a thread
-// (threads per block x blocks per SM: 128 x 5).
+// (threads per block x blocks per SM: 128 x 5, of which shared memory holds four).
 #include <cuda_runtime.h>
 
 #include "kf_kernels.cuh"

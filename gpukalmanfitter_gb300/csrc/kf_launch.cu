@@ -129,11 +129,12 @@ constexpr int64_t kFillWarps = 4;  // one on each SM sub-partition
 // same whatever its active lanes, each SM sub-partition starts one every 64
 // cycles, and four warps (one a sub-partition) fill an SM's FP64 pipe.  So a
 // batch first spreads over 3 warps on every SM with as few tracks a warp as
-// that takes (fewer lanes to wait for: 1000 map tracks mixed 1530 -> 1393
-// us), then over 4 ... 8 of them, the kernel's residency (from 5 on the kernel
-// may take a queue of 4 instead, unevenTracks); beyond that warps of 32
-// tracks claim work from the queue.  Sorting (3 small kernels, 15 us)
-// pays from 8 tracks a warp on.
+// that takes (fewer lanes to wait for: 1000 map tracks mixed, one lane a track,
+// 1530 -> 1393 us; such batches now run eight lanes a track, kCoopMost, and
+// this serves the ones that cannot), then over 4 ... 8 of them, the kernel's
+// residency (from 5 on the kernel may take a queue of 4 instead,
+// unevenTracks); beyond that warps of 32 tracks claim work from the queue.
+// Sorting (3 small kernels, 15 us) pays from 8 tracks a warp on.
 struct Spread {
   int lanes;  // tracks per warp
   bool sort;  // order the tracks by expected work

@@ -133,17 +133,19 @@ typedef struct kf_config {
                                 the smoother takes the reference's general gain
                                 C_f J^T C_p^-1 and the workspace grows (sizes
                                 depend on this field); the batched form runs its
-                                material instantiation (128 threads x 4 CTAs per
-                                SM) whatever the shape fields say */
-  int32_t adjoint_tape;      /* kf_adjoint_batch only: 0 (default) = the forward
-                                records the tape of the whole track (256 doubles
-                                per track and surface, at least 3072); 1 = it
-                                saves checkpoints every 5 measurement states
-                                and the reverse sweep recomputes one 5-state
-                                segment at a time (3072 doubles per track).
-                                The results are bitwise the same; 0 is faster
-                                and is also what a track falls back to 1 from
-                                when its tape runs over */
+                                material kernels, whose launch the batch's size
+                                decides, whatever the shape fields say */
+  int32_t adjoint_tape;      /* kf_adjoint_batch only, the tape's size: 0
+                                (default) = 256 doubles per track and surface,
+                                at least 3072; 1 = 3072 per track.  A track
+                                whose tape runs over has checkpoints every 5
+                                measurement states instead, from which the
+                                reverse sweep recomputes one 5-state segment at
+                                a time; in a field off the z axis mode 1 does
+                                so for every track.  The results are bitwise
+                                the same there, and along z for tracks that
+                                run over in both modes or in neither (else they
+                                agree to rounding); 0 is faster */
 } kf_config_t;
 
 /* The surface sequence: boundless plane surfaces (PlaneSurface<InfiniteBounds>,
@@ -340,8 +342,8 @@ const char *kf_noalloc_last_error_string(void);
  *   - each track's start parameters (perigee d0, z0, phi, theta, q/p, t);
  *   - the field scale (kf_field_t.scale).
  * Supported: cfg->precision FP64, uniform field, faithful_jacobian = 1.
- * The forward states are checkpointed every 5 measurement states and each
- * segment is recomputed during the reverse sweep. */
+ * The forward records a tape, which the reverse sweep reads backwards; a
+ * track whose tape runs over is recomputed in segments (see adjoint_tape). */
 typedef struct kf_adjoint_outputs {
   double *chi2;             /* [n] smoothed chi2 per track (0 unless OK) */
   int32_t *status;          /* [n] kf_track_status */
