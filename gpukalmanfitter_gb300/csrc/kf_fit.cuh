@@ -414,7 +414,9 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT, H> &L, const Para
     y = h * k;
     x = y * y;
     hy = h * y;
-    if (akey(hy * x) <= P.errBound && akey(y) <= 0x3fb999999999999aLL) break;
+    // (a step whose square overflows, towards no plane, is rejected in any field)
+    const bool far = akey(h) > 0x5fefffffffffffffLL;
+    if (akey(hy * x) <= P.errBound && akey(y) <= 0x3fb999999999999aLL && !far) break;
     const double v0 = fma(-y, dx, dy), v1 = fma(-y, dy, -dx);
     double n1;
     if (FORM == kUniformAny)
@@ -422,7 +424,7 @@ __device__ __forceinline__ void stepUniform(FitLane<FORM, MAT, H> &L, const Para
            fabs(P.rot[2] * v0 + P.rot[5] * v1);
     else
       n1 = fabs(v0) + fabs(v1);
-    const double e0 = 0.25 * fabs(hy) * x * n1;
+    const double e0 = far ? DBL_MAX : 0.25 * fabs(hy) * x * n1;
     const double err = e0 < 1e-20 ? 1e-20 : e0;
     if (err <= P.tol) break;
     if (!rejectTrial(L, P, err, h, nTrials)) {
