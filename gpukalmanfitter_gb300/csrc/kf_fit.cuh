@@ -712,7 +712,10 @@ template <bool MAT, class H> __device__ __forceinline__ void rkStep(FitLane<kGri
 __device__ __forceinline__ double trialErrorUniform(const FieldD &F, const double dir[3], double qop,
                                                     double h) {
   kfa::PolyStep w;
-  kfa::polyTrialFwd(dir, qop, h, F.B, w);
+  kfa::polyPrep(dir, F.B, w);
+  // no field: the estimate's floor while h^2 is finite, whatever h q/p is
+  if (w.beta == 0.) return akey(h) > 0x5fefffffffffffffLL ? DBL_MAX : 1e-20;
+  kfa::polyCoef(qop, h, w);
   return w.err;
 }
 static __device__ __noinline__ double trialError(const FieldD &F, double p0, double p1, double p2,
